@@ -272,8 +272,10 @@ extern "C" int telb_gemm_skinny_fused(int kind, const void* x, const void* x_sf,
                                       int* status, int force_ranks, const telb::TelbGemmFusion* fusion, cudaStream_t stream);
 
 extern "C" int telb_nvfp4_wide_mode();
+extern "C" int telb_gemm_nvfp4_tile_launch(const void* xq, const void* x_sf, const void* wq, const void* w_sf, int M, int N, int K,
+                                           const void* params_blob, cudaStream_t stream);
 extern "C" int telb_gemm_nvfp4_wide_launch(const void* xq, const void* x_sf, const void* wq, const void* w_sf, int M, int N, int K,
-                                           const void* params_blob, int pair, cudaStream_t stream);
+                                           const void* params_blob, cudaStream_t stream);
 
 // Number of 64-element K groups the scale buffers are padded to (whole 256-element stages).
 extern "C" int telb_nvfp4_k64_pad(int k);
@@ -348,7 +350,8 @@ static int gemm_nvfp4_impl(const void* xq, const void* x_sf, const void* wq, con
         p.residual = residual;
         p.out_bf16 = out_bf16;
         p.status = status;
-        return telb_gemm_nvfp4_wide_launch(xq, x_sf, wq, w_sf, M, N, K, &p, wide == 2 ? 1 : 0, stream);
+        if (wide == 1) return telb_gemm_nvfp4_tile_launch(xq, x_sf, wq, w_sf, M, N, K, &p, stream);
+        return telb_gemm_nvfp4_wide_launch(xq, x_sf, wq, w_sf, M, N, K, &p, stream);
     }
     p.k = K;
     p.kb_total = (K + kFp4BK - 1) / kFp4BK;

@@ -1,13 +1,10 @@
-// NVFP4 block-scaled GEMM for prefill-size M with 256-wide output tiles, as a single CTA (128 x 256) or as a
-// CTA pair (`tcgen05.mma.cta_group::2`, 256 x 256 per pair):
+// NVFP4 block-scaled GEMM for prefill-size M on a CTA pair (`tcgen05.mma.cta_group::2`, 256 x 256 per pair):
 //     out[M,N] = (xq ⊙ sfx)[M,K] · (wq ⊙ sfw)[N,K]ᵀ · alpha[N]  (+ bias, + residual)
 //
-// Why a second kernel next to gemm_nvfp4_tc5.cu: with 128 x 128 tiles the block-scaled tensor pipe waits for
-// shared memory to fill — a K step of 256 moves 36 KB from L2 per 8.4 MFLOP, which at the fp4 rate asks for
-// more L2 → SM bandwidth than the chip has.  A pair of CTAs on neighbouring SMs that issues one 256 x 256 MMA
-// needs, per CTA and K step, only its own 128 A rows, HALF of the B tile (the tensor cores of both SMs read
-// both halves in place) and the scales: 38 KB per 16.8 MFLOP, 1.9x the arithmetic per byte.  The single-CTA
-// form (54 KB per 16.8 MFLOP) is kept as the fallback when clusters of two cannot be scheduled.
+// A pair of CTAs on neighbouring SMs that issues one 256 x 256 MMA needs, per CTA and K step, only its own 128 A rows, HALF of the B
+// tile (the tensor cores of both SMs read both halves in place) and the scales: 38 KB per 16.8 MFLOP, against 54 KB of the single-CTA
+// kernel (gemm_nvfp4_tile_tc5.cu).  It is selectable but not the default: its scale factors are copied by `tcgen05.cp` in front of
+// the MMAs, which costs more than the smaller traffic gains (8192 x 24576 x 4096: 662 us against 392 us).
 //
 // No TMA load in this file uses cluster multicast (this kernel runs inside tensor-parallel steps at world
 // sizes above one): each CTA fetches its own A rows, its own half of B and its own copy of the scales.  The
@@ -46,16 +43,15 @@ constexpr int kWSf0 = 384;                  // first scale-factor column
 constexpr int kWSfCols = 48;                // SFA 16 + SFB 32 per buffer
 constexpr int kWTmemCols = 512;
 
-template <bool PAIR>
 struct WideCfg {
-    static constexpr int kTileM = PAIR ? 256 : 128;
-    static constexpr int kBRows = PAIR ? 128 : 256;          // B rows one CTA keeps in shared memory
+    static constexpr int kTileM = 256;
+    static constexpr int kBRows = 128;                       // B rows one CTA keeps in shared memory
     static constexpr int kATile = 128 * 128;
     static constexpr int kBTile = kBRows * 128;
     static constexpr int kSfA = 2048;
     static constexpr int kSfB = 4096;
     static constexpr int kStage = kATile + kBTile + kSfA + kSfB;
-    static constexpr int kStages = PAIR ? 5 : 3;
+    static constexpr int kStages = 5;
     static constexpr int kNumBars = 3 * kStages + 6;
     static constexpr int kSmem = kStages * kStage + 1024 + 256 + kRsStageBytes;
 };
@@ -131,12 +127,11 @@ __device__ __forceinline__ WideTile wide_tile(const GemmParams& p, int t) {
     return w;
 }
 
-template <bool PAIR>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                        const __grid_constant__ CUtensorMap tma_sfa, const __grid_constant__ CUtensorMap tma_sfb,
-                       const uint8_t* __restrict__ sf_a, const uint8_t* __restrict__ sf_b, int sf_k64_a, int sf_k64_b, GemmParams p) {
-    using Cfg = WideCfg<PAIR>;
+                       int sf_k64_a, int sf_k64_b, GemmParams p) {
+    using Cfg = WideCfg;
     constexpr int STAGES = Cfg::kStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -152,9 +147,9 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const uint32_t crank = PAIR ? cluster_ctarank_w() : 0u;
+    const uint32_t crank = cluster_ctarank_w();
     const bool leader = crank == 0;
-    const int ncta = PAIR ? 2 : 1;
+    constexpr int ncta = 2;
     const int cid = blockIdx.x / ncta, ncl = gridDim.x / ncta;
     const int total_tiles = p.tiles_a * p.tiles_b;
 
@@ -173,23 +168,16 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
         mbar_fence_init();
         prefetch_tensormap(&tma_a);
         prefetch_tensormap(&tma_b);
-        if constexpr (PAIR) {
-            prefetch_tensormap(&tma_sfa);
-            prefetch_tensormap(&tma_sfb);
-        }
+        prefetch_tensormap(&tma_sfa);
+        prefetch_tensormap(&tma_sfb);
     }
     if (warp == 1) {
-        if constexpr (PAIR) {
-            tmem_alloc2(tmem_slot, kWTmemCols);
-            tmem_relinquish2();
-        } else {
-            tmem_alloc(tmem_slot, kWTmemCols);
-            tmem_relinquish();
-        }
+        tmem_alloc2(tmem_slot, kWTmemCols);
+        tmem_relinquish2();
     }
     tc_fence_before_sync();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync_w();       // both CTAs' barriers and TMEM exist before anything crosses the pair
+    cluster_sync_w();       // both CTAs' barriers and TMEM exist before anything crosses the pair
     tc_fence_after_sync();
     pdl_prologue();
     const uint32_t tmem_base = *tmem_slot;
@@ -205,7 +193,7 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
             for (int t = cid; t < total_tiles && ok; t += ncl) {
                 const WideTile w = wide_tile<Cfg::kTileM>(p, t);
                 const int a0 = w.a0 + (int)crank * 128;
-                const int brow = w.b0 + (PAIR ? (int)crank * 128 : 0);
+                const int brow = w.b0 + (int)crank * 128;
                 if (p.ag_flags && a0 < p.rows_a && !ag_wait_rows(p, a0, ag_e, abort_flag)) break;
                 const int ta = min(a0 / 128, last_a_tile);
                 const int tb0 = min(w.b0 / 128, last_b_tile), tb1 = min(w.b0 / 128 + 1, last_b_tile);
@@ -218,25 +206,16 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     uint8_t* sb = sa + Cfg::kATile;
                     uint8_t* ssa = sb + Cfg::kBTile;
                     uint8_t* ssb = ssa + Cfg::kSfA;
-                    if constexpr (PAIR) {
-                        // every load of both CTAs completes on the LEADER's barrier (armed by the leader for both stages'
-                        // bytes), so the issuer learns that the pair's operands are in place without a relay hop; the scale
-                        // atoms travel as tiled loads too (rows of 512 bytes), since only those can signal the peer's barrier
-                        const uint32_t fb = cluster_addr_of(&full_bar[stage], 0);
-                        if (leader) mbar_expect_tx(&full_bar[stage], 2 * Cfg::kStage);
-                        tma_load_2d_pair(sa, &tma_a, fb, kb * 128, a0);
-                        tma_load_2d_pair(sb, &tma_b, fb, kb * 128, brow);
-                        tma_load_2d_pair(ssa, &tma_sfa, fb, 0, ta * sf_k64_a + kb * 4);
-                        tma_load_2d_pair(ssb, &tma_sfb, fb, 0, tb0 * sf_k64_b + kb * 4);
-                        tma_load_2d_pair(ssb + 2048, &tma_sfb, fb, 0, tb1 * sf_k64_b + kb * 4);
-                    } else {
-                        mbar_expect_tx(&full_bar[stage], Cfg::kStage);
-                        tma_load_2d(sa, &tma_a, &full_bar[stage], kb * 128, a0);
-                        tma_load_2d(sb, &tma_b, &full_bar[stage], kb * 128, brow);
-                        bulk_load(ssa, sf_a + ((size_t)ta * sf_k64_a + (size_t)kb * 4) * 512, 2048, &full_bar[stage]);
-                        bulk_load(ssb, sf_b + ((size_t)tb0 * sf_k64_b + (size_t)kb * 4) * 512, 2048, &full_bar[stage]);
-                        bulk_load(ssb + 2048, sf_b + ((size_t)tb1 * sf_k64_b + (size_t)kb * 4) * 512, 2048, &full_bar[stage]);
-                    }
+                    // every load of both CTAs completes on the LEADER's barrier (armed by the leader for both stages'
+                    // bytes), so the issuer learns that the pair's operands are in place without a relay hop; the scale
+                    // atoms travel as tiled loads too (rows of 512 bytes), since only those can signal the peer's barrier
+                    const uint32_t fb = cluster_addr_of(&full_bar[stage], 0);
+                    if (leader) mbar_expect_tx(&full_bar[stage], 2 * Cfg::kStage);
+                    tma_load_2d_pair(sa, &tma_a, fb, kb * 128, a0);
+                    tma_load_2d_pair(sb, &tma_b, fb, kb * 128, brow);
+                    tma_load_2d_pair(ssa, &tma_sfa, fb, 0, ta * sf_k64_a + kb * 4);
+                    tma_load_2d_pair(ssb, &tma_sfb, fb, 0, tb0 * sf_k64_b + kb * 4);
+                    tma_load_2d_pair(ssb + 2048, &tma_sfb, fb, 0, tb1 * sf_k64_b + kb * 4);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -274,26 +253,18 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     const uint32_t t_sfb = t_sfa + 16;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        if constexpr (PAIR) {
-                            tmem_cp_sf2(t_sfa + q * 4, smem_desc_sf(ssa + q * 512));
-                            tmem_cp_sf2(t_sfb + q * 8, smem_desc_sf(ssb + q * 512));
-                            tmem_cp_sf2(t_sfb + q * 8 + 4, smem_desc_sf(ssb + 2048 + q * 512));
-                        } else {
-                            tmem_cp_sf(t_sfa + q * 4, smem_desc_sf(ssa + q * 512));
-                            tmem_cp_sf(t_sfb + q * 8, smem_desc_sf(ssb + q * 512));
-                            tmem_cp_sf(t_sfb + q * 8 + 4, smem_desc_sf(ssb + 2048 + q * 512));
-                        }
+                        tmem_cp_sf2(t_sfa + q * 4, smem_desc_sf(ssa + q * 512));
+                        tmem_cp_sf2(t_sfb + q * 8, smem_desc_sf(ssb + q * 512));
+                        tmem_cp_sf2(t_sfb + q * 8 + 4, smem_desc_sf(ssb + 2048 + q * 512));
                     }
                     const uint64_t da = smem_desc_sw128(sa);
                     const uint64_t db = smem_desc_sw128(sb);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const uint32_t accum = (kb > 0 || q > 0) ? 1u : 0u;
-                        if constexpr (PAIR) umma_nvfp4_2(d_tmem, da + 2 * q, db + 2 * q, idesc, t_sfa + q * 4, t_sfb + q * 8, accum);
-                        else umma_nvfp4(d_tmem, da + 2 * q, db + 2 * q, idesc, t_sfa + q * 4, t_sfb + q * 8, accum);
+                        umma_nvfp4_2(d_tmem, da + 2 * q, db + 2 * q, idesc, t_sfa + q * 4, t_sfb + q * 8, accum);
                     }
-                    if constexpr (PAIR) umma_commit2(&empty_bar[stage], 3);
-                    else umma_commit(&empty_bar[stage]);
+                    umma_commit2(&empty_bar[stage], 3);
                     sf_par ^= 1;
                     if (++stage == STAGES) {
                         stage = 0;
@@ -301,8 +272,7 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     }
                 }
                 if (!ok) break;
-                if constexpr (PAIR) umma_commit2(&tfull_bar[acc], 3);
-                else umma_commit(&tfull_bar[acc]);
+                umma_commit2(&tfull_bar[acc], 3);
             }
         }
     } else {
@@ -428,11 +398,9 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                 }
                 tc_fence_before_sync();
                 if (hh == 0) {
-                    if constexpr (PAIR) mbar_arrive_cluster(&tovl_bar[acc], 0);
-                    else mbar_arrive(&tovl_bar[acc]);
+                    mbar_arrive_cluster(&tovl_bar[acc], 0);
                 } else {
-                    if constexpr (PAIR) mbar_arrive_cluster(&tempty_bar[acc], 0);
-                    else mbar_arrive(&tempty_bar[acc]);
+                    mbar_arrive_cluster(&tempty_bar[acc], 0);
                 }
             }
         }
@@ -447,54 +415,48 @@ gemm_nvfp4_wide_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     }
     tc_fence_before_sync();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync_w();       // the other CTA's tensor core may still be reading this CTA's tiles / TMEM
+    cluster_sync_w();       // the other CTA's tensor core may still be reading this CTA's tiles / TMEM
     if (warp == 1) {
         tc_fence_after_sync();
-        if constexpr (PAIR) tmem_dealloc2(tmem_base, kWTmemCols);
-        else tmem_dealloc(tmem_base, kWTmemCols);
+        tmem_dealloc2(tmem_base, kWTmemCols);
     }
 }
 
-template <bool PAIR>
-static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsfa, const CUtensorMap& tsfb, const uint8_t* sfa,
-                       const uint8_t* sfb, int k64a, int k64b, const GemmParams& p, cudaStream_t stream) {
-    using Cfg = WideCfg<PAIR>;
-    auto kern = gemm_nvfp4_wide_kernel<PAIR>;
+static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsfa, const CUtensorMap& tsfb, int k64,
+                       const GemmParams& p, cudaStream_t stream) {
+    using Cfg = WideCfg;
+    auto kern = gemm_nvfp4_wide_kernel;
     static int max_clusters = 0;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
         if (e != cudaSuccess) return fail("cudaFuncSetAttribute(gemm_nvfp4_wide)", e);
-        if (PAIR) {
-            // how many pairs can be resident at once: a pair needs two free SMs of one TPC / GPC, so it is queried, not assumed
-            cudaLaunchConfig_t q{};
-            q.gridDim = dim3(sm_count() / 2 * 2, 1, 1);
-            q.blockDim = dim3(kGemmThreads, 1, 1);
-            q.dynamicSmemBytes = Cfg::kSmem;
-            cudaLaunchAttribute a[1];
-            a[0].id = cudaLaunchAttributeClusterDimension;
-            a[0].val.clusterDim.x = 2;
-            a[0].val.clusterDim.y = 1;
-            a[0].val.clusterDim.z = 1;
-            q.attrs = a;
-            q.numAttrs = 1;
-            int n = 0;
-            e = cudaOccupancyMaxActiveClusters(&n, kern, &q);
-            if (e != cudaSuccess || n <= 0) {
-                cudaGetLastError();
-                n = sm_count() / 2;
-            }
-            max_clusters = n;
-            if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", n, sm_count());
-        } else {
-            max_clusters = sm_count();
+        // how many pairs can be resident at once: a pair needs two free SMs of one TPC / GPC, so it is queried, not assumed
+        cudaLaunchConfig_t q{};
+        q.gridDim = dim3(sm_count() / 2 * 2, 1, 1);
+        q.blockDim = dim3(kGemmThreads, 1, 1);
+        q.dynamicSmemBytes = Cfg::kSmem;
+        cudaLaunchAttribute a[1];
+        a[0].id = cudaLaunchAttributeClusterDimension;
+        a[0].val.clusterDim.x = 2;
+        a[0].val.clusterDim.y = 1;
+        a[0].val.clusterDim.z = 1;
+        q.attrs = a;
+        q.numAttrs = 1;
+        int n = 0;
+        e = cudaOccupancyMaxActiveClusters(&n, kern, &q);
+        if (e != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = sm_count() / 2;
         }
+        max_clusters = n;
+        if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", n, sm_count());
         configured = true;
     }
     const int total = p.tiles_a * p.tiles_b;
     const int clusters = total < max_clusters ? total : max_clusters;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(clusters * (PAIR ? 2 : 1), 1, 1);
+    cfg.gridDim = dim3(clusters * 2, 1, 1);
     cfg.blockDim = dim3(kGemmThreads, 1, 1);
     cfg.dynamicSmemBytes = Cfg::kSmem;
     cfg.stream = stream;
@@ -503,16 +465,14 @@ static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[na].val.programmaticStreamSerializationAllowed = 1;
     if (pdl_enabled()) ++na;
-    if (PAIR) {
-        attrs[na].id = cudaLaunchAttributeClusterDimension;
-        attrs[na].val.clusterDim.x = 2;
-        attrs[na].val.clusterDim.y = 1;
-        attrs[na].val.clusterDim.z = 1;
-        ++na;
-    }
+    attrs[na].id = cudaLaunchAttributeClusterDimension;
+    attrs[na].val.clusterDim.x = 2;
+    attrs[na].val.clusterDim.y = 1;
+    attrs[na].val.clusterDim.z = 1;
+    ++na;
     cfg.attrs = attrs;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tsfa, tsfb, sfa, sfb, k64a, k64b, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tsfa, tsfb, k64, k64, p);
     if (e != cudaSuccess) return fail("cudaLaunchKernelEx(gemm_nvfp4_wide)", e);
     return 0;
 }
@@ -521,7 +481,8 @@ static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
 
 using namespace telb;
 
-// Which large-M NVFP4 kernel runs: 0 = 128 x 128 tiles (gemm_nvfp4_tc5.cu), 1 = 128 x 256 single CTA, 2 = 256 x 256 CTA pair.
+// Which large-M NVFP4 kernel runs: 0 = 128 x 128 tiles (gemm_nvfp4_tc5.cu), 1 = 128 x 256 single CTA
+// (gemm_nvfp4_tile_tc5.cu), 2 = 256 x 256 CTA pair.
 // TELB_NVFP4_WIDE overrides the default.
 static int g_wide_mode = -1;
 extern "C" int telb_nvfp4_wide_mode() {
@@ -539,9 +500,9 @@ extern "C" int telb_set_nvfp4_wide_mode(int mode) {
 }
 
 // Large-M layout only (M > 128 is the caller's business; any M works).  `p` arrives with the epilogue / fusion fields set;
-// this fills the tile geometry and launches.  pair = 0 → single CTA, 1 → CTA pair.
+// this fills the tile geometry and launches.
 extern "C" int telb_gemm_nvfp4_wide_launch(const void* xq, const void* x_sf, const void* wq, const void* w_sf, int M, int N, int K,
-                                           const void* params_blob, int pair, cudaStream_t stream) {
+                                           const void* params_blob, cudaStream_t stream) {
     GemmParams p = *static_cast<const GemmParams*>(params_blob);
     if (K % 32) return fail("telb_gemm_nvfp4_wide: K must be a multiple of 32");
     if (N % 8) return fail("telb_gemm_nvfp4_wide: N must be a multiple of 8");
@@ -555,21 +516,17 @@ extern "C" int telb_gemm_nvfp4_wide_launch(const void* xq, const void* x_sf, con
     p.feat_on_lane = 0;
     p.splits = 1;
     p.kb_per_split = p.kb_total;
-    const int tile_m = pair ? 256 : 128;
-    p.tiles_a = (M + tile_m - 1) / tile_m;
+    p.tiles_a = (M + WideCfg::kTileM - 1) / WideCfg::kTileM;
     p.tiles_b = (N + kWBN - 1) / kWBN;
     const int k64 = ((K + 255) / 256) * 4;
     CUtensorMap ta, tb;
     if (make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, M, kbytes, kbytes, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    if (make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, N, kbytes, kbytes, pair ? 128 : 256, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, N, kbytes, kbytes, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     // the pair kernel fetches scale atoms with tiled loads: the scale buffers seen as rows of 512 bytes (128 x u32), four atoms
     // (one 256-element K step of one 128-row tile) per box
-    CUtensorMap tsa = ta, tsb = tb;
-    if (pair) {
-        const uint64_t atoms_a = (uint64_t)((M + 127) / 128) * k64, atoms_b = (uint64_t)((N + 127) / 128) * k64;
-        if (make_tmap_2d(&tsa, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, x_sf, atoms_a, 128, 512, 4, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1;
-        if (make_tmap_2d(&tsb, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w_sf, atoms_b, 128, 512, 4, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1;
-    }
-    return pair ? launch_wide<true>(ta, tb, tsa, tsb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, k64, p, stream)
-                : launch_wide<false>(ta, tb, tsa, tsb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, k64, p, stream);
+    CUtensorMap tsa, tsb;
+    const uint64_t atoms_a = (uint64_t)((M + 127) / 128) * k64, atoms_b = (uint64_t)((N + 127) / 128) * k64;
+    if (make_tmap_2d(&tsa, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, x_sf, atoms_a, 128, 512, 4, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1;
+    if (make_tmap_2d(&tsb, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w_sf, atoms_b, 128, 512, 4, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1;
+    return launch_wide(ta, tb, tsa, tsb, k64, p, stream);
 }
