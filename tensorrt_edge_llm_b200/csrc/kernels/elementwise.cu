@@ -137,13 +137,13 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
 // One CTA per (row, group).
 template <typename T>
 __global__ void gated_group_rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ z, const T* __restrict__ w,
-                                           T* __restrict__ y, int hidden, int gsize, float eps) {
+                                           T* __restrict__ y, int hidden, int gsize, long long ldz, float eps) {
     pdl_prologue();
     __shared__ float red[32];
     const size_t row = blockIdx.x;
     const int g = blockIdx.y;
     const T* xp = x + row * hidden + g * gsize;
-    const T* zp = z + row * hidden + g * gsize;
+    const T* zp = z + row * ldz + g * gsize;
     float ss = 0.f;
     for (int i = threadIdx.x; i < gsize; i += blockDim.x) {
         const float zz = Cvt<T>::to_f(zp[i]);
@@ -157,6 +157,78 @@ __global__ void gated_group_rmsnorm_kernel(const T* __restrict__ x, const T* __r
         const float n = Cvt<T>::to_f(Cvt<T>::from_f(gv * inv));
         y[row * hidden + g * gsize + i] = Cvt<T>::from_f(n * Cvt<T>::to_f(w[g * gsize + i]));
     }
+}
+
+// The same for groups of V x 256 features, one warp each: 16-byte loads, the gated values stay in registers between the sum and the
+// scaling.  Bound by memory: 7300 x 4096, groups of 512: 37 us, 4.9 TB/s (two passes of 2-byte loads, a CTA per group: 127 us).
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+gated_group_rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ z, const T* __restrict__ w, T* __restrict__ y,
+                                long long rows, int hidden, int n_groups, long long ldz, float eps) {
+    pdl_prologue();
+    constexpr int kGroup = V * 256;
+    const long long item = blockIdx.x * 8ll + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const long long row = item / n_groups;
+    const int g = (int)(item - row * n_groups);
+    if (row >= rows) return;
+    const T* xp = x + row * hidden + g * kGroup;
+    const T* zp = z + row * ldz + g * kGroup;
+    Vec8<T> xv[V], zv[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        xv[i].load(xp + (i * 32 + lane) * 8);
+        zv[i].load(zp + (i * 32 + lane) * 8);
+    }
+    float gv[V][8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float zz = zv[i].get(j);
+            gv[i][j] = xv[i].get(j) * (zz / (1.f + __expf(-zz)));
+            ss += gv[i][j] * gv[i][j];
+        }
+    const float inv = rsqrtf(warp_sum(ss) / kGroup + eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        Vec8<T> wv, o;
+        wv.load(w + g * kGroup + (i * 32 + lane) * 8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o.set(j, Cvt<T>::to_f(Cvt<T>::from_f(gv[i][j] * inv)) * wv.get(j));
+        o.store(y + row * hidden + g * kGroup + (i * 32 + lane) * 8);
+    }
+}
+
+// Gated DeltaNet output norm: RMS-normalise each head of D features, scale (rounded as a norm of its own stores it), times silu(z).
+// D / 8 lanes per head.  7300 x 2048: 27 us, in place of a norm and five element-wise passes in 32 bits (200 us).
+template <typename T, int D>
+__global__ void __launch_bounds__(256)
+rmsnorm_gate_kernel(const T* __restrict__ x, const T* __restrict__ z, const T* __restrict__ w, T* __restrict__ y, long long rows,
+                    int heads, long long ldz, float eps) {
+    pdl_prologue();
+    constexpr int kLanes = D / 8;
+    const long long item = (blockIdx.x * 256ll + threadIdx.x) / kLanes;
+    const int l = threadIdx.x % kLanes;
+    const bool on = item < rows * heads;
+    const long long row = on ? item / heads : 0;
+    const int h = on ? (int)(item - row * heads) : 0;
+    Vec8<T> xv, zv, wv, o;
+    xv.load(x + (row * heads + h) * D + l * 8);
+    zv.load(z + row * ldz + h * D + l * 8);
+    wv.load(w + l * 8);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += xv.get(j) * xv.get(j);
+#pragma unroll
+    for (int s = kLanes / 2; s > 0; s >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, s);
+    const float inv = rsqrtf(ss / D + eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float n = Cvt<T>::to_f(Cvt<T>::from_f(xv.get(j) * inv)) * wv.get(j), zz = zv.get(j);
+        o.set(j, Cvt<T>::to_f(Cvt<T>::from_f(n)) * (zz * (1.f / (1.f + expf(-zz)))));
+    }
+    if (on) o.store(y + (row * heads + h) * D + l * 8);
 }
 
 // out[t, i] = silu(in[t, i]) * in[t, inter + i]
@@ -712,14 +784,45 @@ extern "C" int telb_layernorm(const void* x, const void* w, const void* b, void*
     return 0;
 }
 
+// ldz: elements from a row of z to the next one.  A warp per group where the group is 256, 512, 768 or 1024 features in whole 16-byte pieces.
 extern "C" int telb_gated_group_rmsnorm(const void* x, const void* z, const void* w, void* y, long long rows, int hidden,
-                                        int n_groups, float eps, int is_bf16, cudaStream_t stream) {
+                                        int n_groups, long long ldz, float eps, int is_bf16, cudaStream_t stream) {
     if (rows <= 0) return 0;
-    dim3 grid((unsigned)rows, n_groups);
-    DISPATCH_T(is_bf16, {
-        TELB_LAUNCH("gated_group_rmsnorm_kernel", (gated_group_rmsnorm_kernel<T>), dim3(grid), dim3(256), 0, stream, (const T*)x, (const T*)z, (const T*)w, (T*)y, hidden, hidden / n_groups, eps);
-    })
+    const int gsize = hidden / n_groups;
+    const bool wide = hidden % n_groups == 0 && gsize % 256 == 0 && gsize <= 1024 && ldz % 8 == 0 &&
+                      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+    if (wide) {
+        const dim3 grid((unsigned)((rows * n_groups + 7) / 8));
+#define TELB_GGN(V_) TELB_LAUNCH("gated_group_rmsnorm_warp_kernel", (gated_group_rmsnorm_warp_kernel<T, V_>), grid, dim3(256), 0, stream, \
+                                 (const T*)x, (const T*)z, (const T*)w, (T*)y, rows, hidden, n_groups, ldz, eps)
+        DISPATCH_T(is_bf16, {
+            if (gsize == 256) TELB_GGN(1); else if (gsize == 512) TELB_GGN(2); else if (gsize == 768) TELB_GGN(3); else TELB_GGN(4);
+        })
+#undef TELB_GGN
+    } else {
+        dim3 grid((unsigned)rows, n_groups);
+        DISPATCH_T(is_bf16, {
+            TELB_LAUNCH("gated_group_rmsnorm_kernel", (gated_group_rmsnorm_kernel<T>), dim3(grid), dim3(256), 0, stream, (const T*)x, (const T*)z, (const T*)w, (T*)y, hidden, gsize, ldz, eps);
+        })
+    }
     TELB_CHECK_LAUNCH("gated_group_rmsnorm_kernel");
+    return 0;
+}
+
+// x, y [rows, heads, dim], z [rows, heads * dim] of row pitch ldz; dim 64, 128 or 256, everything 16-byte aligned.
+extern "C" int telb_rmsnorm_gate(const void* x, const void* z, const void* w, void* y, long long rows, int heads, int dim, long long ldz,
+                                 float eps, int is_bf16, cudaStream_t stream) {
+    if (rows <= 0 || heads <= 0) return 0;
+    if (dim != 64 && dim != 128 && dim != 256) return fail("telb_rmsnorm_gate: head size must be 64, 128 or 256");
+    if (ldz % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15))
+        return fail("telb_rmsnorm_gate: rows must be 16-byte aligned");
+    const int per = 256 / (dim / 8);
+    const dim3 grid((unsigned)((rows * heads + per - 1) / per));
+#define TELB_RG(D_) TELB_LAUNCH("rmsnorm_gate_kernel", (rmsnorm_gate_kernel<T, D_>), grid, dim3(256), 0, stream, (const T*)x, (const T*)z, \
+                                (const T*)w, (T*)y, rows, heads, ldz, eps)
+    DISPATCH_T(is_bf16, { if (dim == 64) TELB_RG(64); else if (dim == 128) TELB_RG(128); else TELB_RG(256); })
+#undef TELB_RG
+    TELB_CHECK_LAUNCH("rmsnorm_gate_kernel");
     return 0;
 }
 

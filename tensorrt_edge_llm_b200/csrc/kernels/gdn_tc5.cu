@@ -466,19 +466,19 @@ using namespace telb;
 
 // Gated DeltaNet chunked prefill (see the top of the file).  q, k [T, hk, 128], v [T, hv, 128], a, b [T, hv] 16-bit,
 // A_log / dt_bias [hv] fp32, state [rows, hv, 128, 128] fp32 (read when past_len > 0, always written), out [T, hv, 128].
-// One CTA per (sequence, value head).
+// ldq / ldk / ldv: elements from a row to the next (multiples of 8).  One CTA per (sequence, value head).
 extern "C" int telb_gdn_chunk_prefill(const void* q, const void* k, const void* v, const void* a, const void* b, const float* A_log,
                                       const float* dt_bias, float* state, void* out, const int* q_start, const int* q_len,
                                       const int* past_len, const int* slot_ids, int num_seqs, int total_tokens, int hk, int hv, int kdim,
-                                      int vdim, int is_bf16, int* status, cudaStream_t stream) {
+                                      int vdim, int is_bf16, int* status, long long ldq, long long ldk, long long ldv, cudaStream_t stream) {
     if (num_seqs <= 0 || total_tokens <= 0) return 0;
     if (kdim != 128 || vdim != 128) return fail("telb_gdn_chunk_prefill: key / value head dims of 128 are the compiled shape");
     if (hk <= 0 || hv % hk) return fail("telb_gdn_chunk_prefill: value heads must be a multiple of key heads");
     const CUtensorMapDataType dtp = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     CUtensorMap tq, tk, tv;
-    if (make_tmap_2d(&tq, dtp, 2, q, total_tokens, (uint64_t)hk * 128, (uint64_t)hk * 256, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    if (make_tmap_2d(&tk, dtp, 2, k, total_tokens, (uint64_t)hk * 128, (uint64_t)hk * 256, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    if (make_tmap_2d(&tv, dtp, 2, v, total_tokens, (uint64_t)hv * 128, (uint64_t)hv * 256, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tq, dtp, 2, q, total_tokens, (uint64_t)hk * 128, (uint64_t)ldq * 2, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tk, dtp, 2, k, total_tokens, (uint64_t)hk * 128, (uint64_t)ldk * 2, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tv, dtp, 2, v, total_tokens, (uint64_t)hv * 128, (uint64_t)ldv * 2, kGdnL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     GdnParams p{};
     p.a = a;
     p.b = b;

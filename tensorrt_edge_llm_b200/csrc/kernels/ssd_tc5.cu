@@ -34,18 +34,19 @@ constexpr int kSsdN = 128;        // state size
 constexpr int kSsdThreads = 192;
 
 struct SsdParams {
-    const void* dt;            // [T, nh]
-    const float* A;            // [nh] (negative)
+    const void* dt;            // [T, nh], row pitch ld_dt
+    const float* A;            // [nh] (negative), or its logarithm without the sign where a_log is set
     const float* D;            // [nh]
     const float* dt_bias;      // [nh]
-    const void* z;             // [T, nh, 64] or null
+    const void* z;             // [T, nh, 64] or null, row pitch ld_z
     float* state;              // [rows, nh, 64, 128] fp32
     void* y;                   // [T, nh, 64]
     const int* q_start;
     const int* q_len;
     const int* past_len;
     const int* slot_ids;
-    int nheads, ngroups, dt_softplus;
+    int nheads, ngroups, dt_softplus, a_log;
+    long long ld_dt, ld_z;     // elements from a row to the next
     float dt_limit;
     int* status;
 };
@@ -172,7 +173,7 @@ ssd_chunk_scan_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
         const int quad = warp & 3;
         const int r = quad * 32 + lane;
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-        const float a_head = p.A[h], d_head = p.D[h], db = p.dt_bias[h];
+        const float a_head = p.a_log ? -(float)exp((double)p.A[h]) : p.A[h], d_head = p.D[h], db = p.dt_bias[h];
         const T* dtp = reinterpret_cast<const T*>(p.dt);
         const T* zp = reinterpret_cast<const T*>(p.z);
         T* yp = reinterpret_cast<T*>(p.y);
@@ -209,7 +210,7 @@ ssd_chunk_scan_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
             // ---- dt, cumulative decay exponent (base-2) ----
             float d = 0.f;
             if (valid) {
-                d = Cvt<T>::to_f(dtp[t * p.nheads + h]) + db;
+                d = Cvt<T>::to_f(dtp[t * p.ld_dt + h]) + db;
                 if (p.dt_softplus) d = ssd_softplus(d);
                 if (p.dt_limit > 0.f) d = fminf(d, p.dt_limit);
             }
@@ -278,7 +279,7 @@ ssd_chunk_scan_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
                 }
                 if (valid) {
                     if (zp) {
-                        const uint4 zu = *reinterpret_cast<const uint4*>(zp + (t * p.nheads + h) * kSsdP + c8 * 8);
+                        const uint4 zu = *reinterpret_cast<const uint4*>(zp + t * p.ld_z + h * kSsdP + c8 * 8);
                         const T* ze = reinterpret_cast<const T*>(&zu);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -364,22 +365,25 @@ using namespace telb;
 
 // Mamba2 chunked prefill scan (see the top of the file).  x [T, nh, 64], dt [T, nh], B / C [T, ngroups, 128] 16-bit,
 // A / D / dt_bias [nh] fp32, z [T, nh, 64] or null, state [rows, nh, 64, 128] fp32 (read when past_len > 0, always
-// written), y [T, nh, 64].  One CTA per (sequence, head).
+// written), y [T, nh, 64].  pitch: elements from a row to the next of x, dt, B, C, z (those of x, B, C multiples of 8).  One CTA per (sequence, head).
 extern "C" int telb_ssd_chunk_scan(const void* x, const void* dt, const float* A, const void* B, const void* C, const float* D,
                                    const float* dt_bias, const void* z, float* state, void* y, const int* q_start, const int* q_len,
                                    const int* past_len, const int* slot_ids, int num_seqs, int total_tokens, int nheads, int head_dim,
                                    int d_state, int ngroups, int dt_softplus, float dt_limit, int is_bf16, int* status,
-                                   cudaStream_t stream) {
+                                   const long long* pitch, int a_log, cudaStream_t stream) {
     if (num_seqs <= 0 || total_tokens <= 0) return 0;
     if (head_dim != kSsdP || d_state != kSsdN) return fail("telb_ssd_chunk_scan: head_dim 64 and d_state 128 are the compiled shape");
     if (ngroups <= 0 || nheads % ngroups) return fail("telb_ssd_chunk_scan: heads must divide evenly into groups");
     const CUtensorMapDataType dtp = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     CUtensorMap tx, tb, tc;
-    if (make_tmap_2d(&tx, dtp, 2, x, total_tokens, (uint64_t)nheads * kSsdP, (uint64_t)nheads * kSsdP * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    if (make_tmap_2d(&tb, dtp, 2, B, total_tokens, (uint64_t)ngroups * kSsdN, (uint64_t)ngroups * kSsdN * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    if (make_tmap_2d(&tc, dtp, 2, C, total_tokens, (uint64_t)ngroups * kSsdN, (uint64_t)ngroups * kSsdN * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tx, dtp, 2, x, total_tokens, (uint64_t)nheads * kSsdP, (uint64_t)pitch[0] * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tb, dtp, 2, B, total_tokens, (uint64_t)ngroups * kSsdN, (uint64_t)pitch[2] * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tc, dtp, 2, C, total_tokens, (uint64_t)ngroups * kSsdN, (uint64_t)pitch[3] * 2, kSsdL, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     SsdParams p{};
     p.dt = dt;
+    p.a_log = a_log;
+    p.ld_dt = pitch[1];
+    p.ld_z = pitch[4];
     p.A = A;
     p.D = D;
     p.dt_bias = dt_bias;

@@ -170,13 +170,13 @@ class MambaMixer(nn.Module):
         z, xbc, dt = proj.split([self.d_inner, self.d_inner + 2 * self.bc, self.nheads], dim=-1)
         if state.record is not None:
             state.record[layer_idx] = (xbc.contiguous(), dt.contiguous())
-        xbc = ops.causal_conv1d(xbc.contiguous(), self.conv_weight, self.conv_bias, state.conv[layer_idx], meta, activation=True)
+        xbc = ops.causal_conv1d(xbc, self.conv_weight, self.conv_bias, state.conv[layer_idx], meta, activation=True)
         xs, B, C = xbc.split([self.d_inner, self.bc, self.bc], dim=-1)
         t = x.shape[0]
-        y = ops.ssm_scan(xs.reshape(t, self.nheads, m.head_dim), dt.contiguous(), -torch.exp(self.A_log),
+        y = ops.ssm_scan(xs.reshape(t, self.nheads, m.head_dim), dt, self.A_log,
                          B.reshape(t, self.groups, m.d_state), C.reshape(t, self.groups, m.d_state), self.D, self.dt_bias,
-                         state.ssm[layer_idx], meta, z=None, dt_softplus=True, dt_limit=m.dt_limit)
-        y = ops.gated_group_rmsnorm(y.reshape(t, self.d_inner), z.contiguous(), self.norm_weight, self.groups, self.eps)
+                         state.ssm[layer_idx], meta, z=None, dt_softplus=True, dt_limit=m.dt_limit, a_log=True)
+        y = ops.gated_group_rmsnorm(y.reshape(t, self.d_inner), z, self.norm_weight, self.groups, self.eps)
         return self.out_proj(y)
 
 
@@ -188,9 +188,9 @@ class MambaMixer(nn.Module):
         xbc = ops.causal_conv1d(xbc, self.conv_weight, self.conv_bias, state.conv[layer_idx], meta, activation=True)
         xs, B, C = xbc.split([self.d_inner, self.bc, self.bc], dim=-1)
         t = xbc.shape[0]
-        ops.ssm_scan(xs.reshape(t, self.nheads, m.head_dim), dt, -torch.exp(self.A_log), B.reshape(t, self.groups, m.d_state),
+        ops.ssm_scan(xs.reshape(t, self.nheads, m.head_dim), dt, self.A_log, B.reshape(t, self.groups, m.d_state),
                      C.reshape(t, self.groups, m.d_state), self.D, self.dt_bias, state.ssm[layer_idx], meta, z=None, dt_softplus=True,
-                     dt_limit=m.dt_limit)
+                     dt_limit=m.dt_limit, a_log=True)
 
 
 class GatedDeltaNetMixer(nn.Module):
@@ -255,10 +255,7 @@ class GatedDeltaNetMixer(nn.Module):
         o = ops.gated_delta_rule(q.reshape(t, self.hk, g.head_k_dim), k.reshape(t, self.hk, g.head_k_dim),
                                  v.reshape(t, self.hv, g.head_v_dim), a, b, self.A_log, self.dt_bias, state.gdn[layer_idx], meta)
         # per-head RMSNorm, then the silu(z) gate
-        o = ops.rmsnorm(o.reshape(t * self.hv, g.head_v_dim).contiguous(), self.norm_weight, self.eps).reshape(t, self.value_dim)
-        zf = z.float()
-        o = (o.float() * (zf * torch.sigmoid(zf))).to(x.dtype)
-        return self.out_proj(o)
+        return self.out_proj(ops.rmsnorm_gate(o, z, self.norm_weight, self.eps))
 
 
     @torch.no_grad()

@@ -60,6 +60,12 @@ def gated_group_rmsnorm(x, z, weight, n_groups, eps):
     return ref.gated_group_rmsnorm(x, z, weight, n_groups, eps)
 
 
+def rmsnorm_gate(x, z, weight, eps):
+    if x.is_cuda:
+        return cuda_ops().rmsnorm_gate(x, z, weight, eps)
+    return ref.rmsnorm_gate(x, z, weight, eps)
+
+
 def swiglu(gate_up, quant_scale=None, interleaved=False):
     """``interleaved``: the columns hold blocks of 64 gate features followed by their 64 up features (the layout the fused
     gate/up GEMM epilogue uses) instead of ``[gate | up]``; only the quantising CUDA form takes it."""
@@ -390,10 +396,10 @@ def causal_conv1d(x, weight, bias, conv_state, meta, activation=True):
     return ref.causal_conv1d(x, weight, bias, conv_state, meta, activation)
 
 
-def ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z=None, dt_softplus=True, dt_limit=0.0):
+def ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z=None, dt_softplus=True, dt_limit=0.0, a_log=False):
     if x.is_cuda:
-        return cuda_ops().ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z, dt_softplus, dt_limit)
-    return ref.ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z, dt_softplus, dt_limit)
+        return cuda_ops().ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z, dt_softplus, dt_limit, a_log)
+    return ref.ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta, z, dt_softplus, dt_limit, a_log)
 
 
 def gated_delta_rule(q, k, v, a, b, A_log, dt_bias, state, meta):

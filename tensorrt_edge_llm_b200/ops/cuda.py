@@ -164,12 +164,39 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
     return y
 
 
+def _rows(t: torch.Tensor):
+    """``(tensor, elements from a row to the next)`` of rows ``[T, ...]`` that a kernel reads by 16-byte pieces where they lie: a view into
+    wider rows stays one where each row is packed and starts on 16 bytes; everything else is copied."""
+    if t.is_contiguous():
+        return t, t.stride(0) if t.dim() > 1 and t.shape[0] > 1 else t[0].numel() if t.shape[0] else 0
+    packed = t.shape[0] > 0 and t[0].is_contiguous() and t.stride(0) >= t[0].numel()
+    if not packed or (t.stride(0) * t.element_size()) % 16 or t.data_ptr() % 16:
+        t = t.contiguous()
+    return t, t.stride(0)
+
+
 def gated_group_rmsnorm(x, z, weight, n_groups, eps):
-    x, z = x.contiguous(), z.contiguous()
+    x = x.contiguous()
     y = torch.empty_like(x)
     rows = x.numel() // x.shape[-1]
+    z, ldz = _rows(z.reshape(rows, x.shape[-1]))
     _check(lib().telb_gated_group_rmsnorm(_p(x), _p(z), _p(weight), _p(y), c_ll(rows), c_int(x.shape[-1]),
-                                          c_int(n_groups), c_float(eps), c_int(_is_bf16(x)), _stream()), "gated_group_rmsnorm")
+                                          c_int(n_groups), c_ll(ldz), c_float(eps), c_int(_is_bf16(x)), _stream()), "gated_group_rmsnorm")
+    return y
+
+
+def rmsnorm_gate(x, z, weight, eps):
+    """RMS norm of every head of ``x [T, heads, dim]``, times ``silu(z [T, heads * dim])``: ``[T, heads * dim]``."""
+    t, heads, dim = x.shape
+    if dim not in (64, 128, 256):
+        n = rmsnorm(x.reshape(t * heads, dim).contiguous(), weight, eps).reshape(t, heads * dim)
+        zf = z.float()
+        return (n.float() * (zf * torch.sigmoid(zf))).to(x.dtype)
+    x = x.contiguous()
+    z, ldz = _rows(z)
+    y = torch.empty(t, heads * dim, dtype=x.dtype, device=x.device)
+    _check(lib().telb_rmsnorm_gate(_p(x), _p(z), _p(weight), _p(y), c_ll(t), c_int(heads), c_int(dim), c_ll(ldz), c_float(eps),
+                                   c_int(_is_bf16(x)), _stream()), "rmsnorm_gate")
     return y
 
 
@@ -1104,14 +1131,14 @@ def moe_combine(y: torch.Tensor, ws, topk_w: torch.Tensor, out: Optional[torch.T
 
 
 def causal_conv1d(x, weight, bias, conv_state, meta: StepMeta, activation=True):
-    x = x.contiguous()
+    x, ldx = _rows(x)
     t, c = x.shape
     w = weight.reshape(c, -1).contiguous()
-    out = torch.empty_like(x)
+    out = torch.empty(t, c, dtype=x.dtype, device=x.device)
     assert conv_state.is_contiguous() and conv_state.dtype == x.dtype
     _check(lib().telb_causal_conv1d(_p(x), _p(w), _p(bias), _p(conv_state), _p(out), _p(meta.seq_ids), _p(meta.q_start),
                                     _p(meta.q_len), _p(meta.past_len), _p(meta.slot_ids), c_int(t), c_int(meta.num_seqs), c_int(c),
-                                    c_int(w.shape[1]), c_int(int(activation)), c_int(_is_bf16(x)), _stream()), "causal_conv1d", 2)
+                                    c_ll(ldx), c_int(w.shape[1]), c_int(int(activation)), c_int(_is_bf16(x)), _stream()), "causal_conv1d", 2)
     return out
 
 
@@ -1121,19 +1148,22 @@ _SSM_SCRATCH = {}
 SSD_TC_MIN_Q = 64        # steps whose longest sequence has at least this many new rows take the tensor-core chunk scan
 
 
-def ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta: StepMeta, z=None, dt_softplus=True, dt_limit=0.0):
-    x, dt, B, C = x.contiguous(), dt.contiguous(), B.contiguous(), C.contiguous()
+def ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta: StepMeta, z=None, dt_softplus=True, dt_limit=0.0, a_log=False):
+    """``a_log``: ``A`` is given as ``log(-A)``, as checkpoints keep it."""
+    (x, ldx), (dt, lddt), (B, ldb), (C, ldc) = _rows(x), _rows(dt), _rows(B), _rows(C)
+    z, ldz = _rows(z) if z is not None else (None, 0)
+    pitch = (c_ll * 5)(ldx, lddt, ldb, ldc, ldz)
     t, nh, hd = x.shape
-    y = torch.empty_like(x)
+    y = torch.empty(t, nh, hd, dtype=x.dtype, device=x.device)
     assert ssm_state.dtype == torch.float32 and ssm_state.is_contiguous()
     if (meta.max_q_len >= SSD_TC_MIN_Q and hd == 64 and B.shape[-1] == 128 and os.environ.get("TELB_DISABLE_SSD_TC", "0") != "1"):
         # prefill: chunked state-space-duality scan on the tensor cores (csrc/kernels/ssd_tc5.cu)
         ws = Workspace.get(x.device)
         _check(lib().telb_ssd_chunk_scan(_p(x), _p(dt), _p(A.float().contiguous()), _p(B), _p(C), _p(D.float().contiguous()),
-                                         _p(dt_bias.float().contiguous()), _p(z.contiguous() if z is not None else None), _p(ssm_state), _p(y),
+                                         _p(dt_bias.float().contiguous()), _p(z), _p(ssm_state), _p(y),
                                          _p(meta.q_start), _p(meta.q_len), _p(meta.past_len), _p(meta.slot_ids), c_int(meta.num_seqs), c_int(t),
                                          c_int(nh), c_int(hd), c_int(B.shape[-1]), c_int(B.shape[1]), c_int(int(dt_softplus)),
-                                         c_float(dt_limit), c_int(_is_bf16(x)), _p(ws.status), _stream()), "ssd_chunk_scan")
+                                         c_float(dt_limit), c_int(_is_bf16(x)), _p(ws.status), pitch, c_int(int(a_log)), _stream()), "ssd_chunk_scan")
         return y
     scratch = None
     if meta.max_q_len >= 256:       # long prefill chunk: parallel segments need per-segment states (see recurrent.cu)
@@ -1143,11 +1173,11 @@ def ssm_scan(x, dt, A, B, C, D, dt_bias, ssm_state, meta: StepMeta, z=None, dt_s
         if scratch is None or scratch.numel() < need:
             scratch = _SSM_SCRATCH[x.device] = torch.empty(need, dtype=torch.float32, device=x.device)
     _check(lib().telb_ssm_scan(_p(x), _p(dt), _p(A.float().contiguous()), _p(B), _p(C), _p(D.float().contiguous()),
-                               _p(dt_bias.float().contiguous()), _p(z.contiguous() if z is not None else None), _p(ssm_state), _p(y),
+                               _p(dt_bias.float().contiguous()), _p(z), _p(ssm_state), _p(y),
                                _p(meta.q_start), _p(meta.q_len), _p(meta.past_len), _p(meta.slot_ids), c_int(meta.num_seqs),
                                c_int(nh), c_int(hd), c_int(B.shape[-1]), c_int(B.shape[1]), c_int(int(dt_softplus)),
                                c_float(dt_limit), c_int(_is_bf16(x)), c_int(meta.max_q_len), _p(scratch),
-                               c_ll(scratch.numel() if scratch is not None else 0), _stream()), "ssm_scan", 3 if scratch is not None else 1)
+                               c_ll(scratch.numel() if scratch is not None else 0), pitch, c_int(int(a_log)), _stream()), "ssm_scan", 3 if scratch is not None else 1)
     return y
 
 
@@ -1155,8 +1185,9 @@ GDN_TC_MIN_Q = 32        # steps whose longest sequence has at least this many n
 
 
 def gated_delta_rule(q, k, v, a, b, A_log, dt_bias, state, meta: StepMeta):
-    q, k, v, a, b = (t.contiguous() for t in (q, k, v, a, b))
-    out = torch.empty_like(v)
+    (q, ldq), (k, ldk), (v, ldv) = _rows(q), _rows(k), _rows(v)
+    a, b = a.contiguous(), b.contiguous()
+    out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
     assert state.dtype == torch.float32 and state.is_contiguous()
     if (meta.max_q_len >= GDN_TC_MIN_Q and q.shape[2] == 128 and v.shape[2] == 128 and os.environ.get("TELB_DISABLE_GDN_TC", "0") != "1"):
         # prefill: chunked (64-token) delta rule with the matrix products on the tensor cores (csrc/kernels/gdn_tc5.cu)
@@ -1164,12 +1195,12 @@ def gated_delta_rule(q, k, v, a, b, A_log, dt_bias, state, meta: StepMeta):
         _check(lib().telb_gdn_chunk_prefill(_p(q), _p(k), _p(v), _p(a), _p(b), _p(A_log.float().contiguous()), _p(dt_bias.float().contiguous()),
                                             _p(state), _p(out), _p(meta.q_start), _p(meta.q_len), _p(meta.past_len), _p(meta.slot_ids),
                                             c_int(meta.num_seqs), c_int(q.shape[0]), c_int(q.shape[1]), c_int(v.shape[1]), c_int(q.shape[2]),
-                                            c_int(v.shape[2]), c_int(_is_bf16(q)), _p(ws.status), _stream()), "gdn_chunk_prefill")
+                                            c_int(v.shape[2]), c_int(_is_bf16(q)), _p(ws.status), c_ll(ldq), c_ll(ldk), c_ll(ldv), _stream()), "gdn_chunk_prefill")
         return out
     _check(lib().telb_gated_delta_rule(_p(q), _p(k), _p(v), _p(a), _p(b), _p(A_log.float().contiguous()),
                                        _p(dt_bias.float().contiguous()), _p(state), _p(out), _p(meta.q_start), _p(meta.q_len),
                                        _p(meta.past_len), _p(meta.slot_ids), c_int(meta.num_seqs), c_int(q.shape[1]), c_int(v.shape[1]),
-                                       c_int(q.shape[2]), c_int(v.shape[2]), c_int(_is_bf16(q)), _stream()), "gated_delta_rule")
+                                       c_int(q.shape[2]), c_int(v.shape[2]), c_int(_is_bf16(q)), c_ll(ldq), c_ll(ldk), c_ll(ldv), _stream()), "gated_delta_rule")
     return out
 
 

@@ -52,6 +52,13 @@ def gated_group_rmsnorm(x: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, 
     return (g.reshape(shp).to(x.dtype).float() * weight.float()).to(x.dtype)
 
 
+def rmsnorm_gate(x: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """RMS norm of every head of ``x [T, heads, dim]``, then times ``silu(z [T, heads * dim])``."""
+    n = rmsnorm(x, weight, eps).reshape(z.shape).float()
+    zf = z.float()
+    return (n * (zf * torch.sigmoid(zf))).to(x.dtype)
+
+
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` where the last dim holds ``[gate | up]`` halves."""
     g, u = gate_up.float().chunk(2, dim=-1)
@@ -498,15 +505,16 @@ def causal_conv1d(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
 
 def ssm_scan(x: torch.Tensor, dt: torch.Tensor, A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, D: torch.Tensor,
              dt_bias: torch.Tensor, ssm_state: torch.Tensor, meta: StepMeta, z: Optional[torch.Tensor] = None,
-             dt_softplus: bool = True, dt_limit: float = 0.0) -> torch.Tensor:
+             dt_softplus: bool = True, dt_limit: float = 0.0, a_log: bool = False) -> torch.Tensor:
     """Mamba2 selective-state recurrence over packed rows (sequential, fp32).
 
-    ``x [T,nh,hd]``, ``dt [T,nh]``, ``A [nh]`` (negative), ``B,C [T,G,N]``, ``D [nh]``,
+    ``x [T,nh,hd]``, ``dt [T,nh]``, ``A [nh]`` (negative; ``log(-A)`` with ``a_log``), ``B,C [T,G,N]``, ``D [nh]``,
     ``ssm_state [rows, nh, hd, N]`` fp32 updated in place; returns ``y [T,nh,hd]``."""
     t, nh, hd = x.shape
     g = B.shape[1]
     hpg = nh // g
-    out = torch.empty_like(x)
+    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    A = -torch.exp(A.float()) if a_log else A
     for s in range(meta.num_seqs):
         r0, ql, past, slot = int(meta.q_start[s]), int(meta.q_len[s]), int(meta.past_len[s]), int(meta.slot_ids[s])
         if ql == 0:

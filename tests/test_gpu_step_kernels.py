@@ -74,3 +74,66 @@ def test_gemm_nvfp4_tile_swiglu_equals_the_128_wide_kernel(cu, m, inter, k, dtyp
     one = torch.full((eye.shape[0],), 1.0, device="cuda") * wi_gs
     rows = [cu.gemm_nvfp4(o.xq, o.sf, wi, cu.nvfp4_swizzle_scales(wi_sf), one, dtype) for o in outs]      # the scales, read as a GEMM reads them
     assert torch.equal(rows[0], rows[1])
+
+
+def _step_meta(q_lens, pasts):
+    from tensorrt_edge_llm_b200.ops import build_step_meta
+    return build_step_meta(q_lens, pasts, torch.zeros(len(q_lens), 1, dtype=torch.int32), 64, slot_ids=list(range(len(q_lens)))[::-1]).to("cuda")
+
+
+@pytest.mark.parametrize("width", [2, 3, 4])
+@pytest.mark.parametrize("channels,ld", [(24, 40), (1040, 1040), (136, 137), (33, 33)])
+@pytest.mark.parametrize("q_lens,pasts", [([1, 1, 1], [5, 0, 9]), ([2, 0, 17, 1, 33], [0, 3, 4, 1, 0]), ([4100], [7])])
+def test_causal_conv1d_of_rows_in_wider_rows(cu, q_lens, pasts, channels, ld, width):
+    """Every rows-per-thread split, sequences that end inside a thread's rows, a pitch that no 16-byte load fits, odd channels."""
+    g = torch.Generator(device="cuda").manual_seed(channels + width)
+    t = sum(q_lens)
+    x = torch.randn(t, ld, device="cuda", generator=g).bfloat16()[:, ld - channels:]
+    w, b = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((channels, width), (channels,)))
+    st = torch.randn(len(q_lens), channels, width - 1, device="cuda", generator=g).bfloat16()
+    st_ref, meta = st.clone(), _step_meta(q_lens, pasts)
+    y, yr = cu.causal_conv1d(x, w, b, st, meta, True), ref.causal_conv1d(x, w, b, st_ref, meta, True)
+    _check_status(cu)
+    # one 16-bit rounding each side, fp32 sums of at most 5 terms
+    assert (y.float() - yr.float()).abs().max() <= 2 ** -7 * yr.float().abs().max() and torch.equal(st, st_ref)
+
+
+@pytest.mark.parametrize("hidden,groups", [(512, 2), (1024, 2), (768, 1), (1024, 1), (96, 3)])
+@pytest.mark.parametrize("rows", [1, 9])
+def test_gated_norms_of_rows_in_wider_rows(cu, rows, hidden, groups):
+    g = torch.Generator(device="cuda").manual_seed(hidden + rows)
+    x, z, w = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((rows, hidden), (rows, hidden + 24), (hidden,)))
+    z = z[:, 8:8 + hidden]
+    y, yr = cu.gated_group_rmsnorm(x, z, w, groups, 1e-5), ref.gated_group_rmsnorm(x, z, w, groups, 1e-5)
+    assert (y.float() - yr.float()).norm() < 2 ** -7 * yr.float().norm()        # two 16-bit roundings
+    for dim in (64, 128, 256, 32):
+        if hidden % dim == 0:
+            h = x.view(rows, hidden // dim, dim)
+            y, yr = cu.rmsnorm_gate(h, z, w[:dim], 1e-5), ref.rmsnorm_gate(h, z, w[:dim], 1e-5)
+            assert (y.float() - yr.float()).norm() < 2 ** -7 * yr.float().norm()
+    _check_status(cu)
+
+
+@pytest.mark.parametrize("q_lens,pasts", [([1, 1, 1], [5, 0, 9]), ([3, 1], [0, 4]), ([37, 130], [0, 64]), ([300], [2])])
+def test_recurrences_read_parts_of_wider_rows(cu, q_lens, pasts):
+    """x, B, C (q, k, v) and the step sizes as views into one projection's rows give the bits of packed copies."""
+    g = torch.Generator(device="cuda").manual_seed(sum(q_lens))
+    t, meta = sum(q_lens), _step_meta(q_lens, pasts)
+    r = torch.randn(t, 4 * 64 + 2 * 256 + 16, device="cuda", generator=g).bfloat16()
+    xs, B, C = r[:, :256].reshape(t, 4, 64), r[:, 256:512].reshape(t, 2, 128), r[:, 512:768].reshape(t, 2, 128)
+    dt, A = r[:, 768:772], torch.rand(4, device="cuda", generator=g)
+    st = torch.randn(len(q_lens), 4, 64, 128, device="cuda", generator=g)
+    D, db = torch.ones(4, device="cuda"), torch.zeros(4, device="cuda")
+    st2 = st.clone()
+    y = cu.ssm_scan(xs, dt, A, B, C, D, db, st, meta, a_log=True)
+    y2 = cu.ssm_scan(xs.contiguous(), dt.contiguous(), -torch.exp(A.double()).float(), B.contiguous(), C.contiguous(), D, db, st2, meta)
+    assert torch.equal(y, y2) and torch.equal(st, st2)
+    r = torch.randn(t, 6 * 128, device="cuda", generator=g).bfloat16()
+    q, k, v = (r[:, i * 256:(i + 1) * 256].reshape(t, 2, 128) for i in range(3))
+    a, b = torch.randn(2, t, 2, device="cuda", generator=g).bfloat16()
+    st = torch.randn(len(q_lens), 2, 128, 128, device="cuda", generator=g) * 0.1
+    st2 = st.clone()
+    y = cu.gated_delta_rule(q, k, v, a, b, A[:2], db[:2], st, meta)
+    y2 = cu.gated_delta_rule(q.contiguous(), k.contiguous(), v.contiguous(), a, b, A[:2], db[:2], st2, meta)
+    assert torch.equal(y, y2) and torch.equal(st, st2)
+    _check_status(cu)
