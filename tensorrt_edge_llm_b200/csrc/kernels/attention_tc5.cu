@@ -146,6 +146,11 @@ extern "C" int telb_attn_combine_dense(const float* ws_o, const float* ws_lse, v
     return 0;
 }
 
+extern "C" int telb_paged_attention_wide(const void* q, const void* kv_layer, void* out, const int* q_start, const int* q_len,
+                                         const int* past_len, const int* page_table, const int* tree_mask, int mask_words, int num_seqs,
+                                         int total_tokens, int num_pages, int max_pages, int page_size, int hq, int hkv, float scale,
+                                         int window, int splits, float* ws, long long ws_floats, int is_bf16, int* status, cudaStream_t stream);
+
 // The dense path (head_dim 64 / 128, no sinks, no skip-softmax); the public entry point telb_paged_attention lives in
 // attention_tc5_extra.cu and forwards here when a step needs none of the extras.  The plain kernel has a translation unit of
 // its own on purpose: sharing one with the extra instantiations cost it 17 % (175 -> 202 us at 8 x 1024 tokens).
@@ -156,13 +161,17 @@ extern "C" int telb_paged_attention_dense(const void* q, const void* kv_layer, v
                                     const int* tree_mask, int mask_words, int num_seqs, int total_tokens,
                                     int max_q_len, int num_pages, int max_pages, int page_size, int hq, int hkv, int d,
                                     float scale, int window, int splits, float* ws, long long ws_floats, int is_bf16,
-                                    int* status, cudaStream_t stream) {
+                                    int* status, int wide, cudaStream_t stream) {
     if (num_seqs <= 0 || total_tokens <= 0) return 0;
     if (d != 64 && d != 128) return fail("telb_paged_attention: head_dim must be 64 or 128 on the dense path");
     if (page_size != 64 && page_size != 128) return fail("telb_paged_attention: page size must be 64 or 128");
     if (hq % hkv) return fail("telb_paged_attention: Hq must be a multiple of Hkv");
     const int group = hq / hkv;
     if (group > 128 || (128 % group)) return fail("telb_paged_attention: GQA ratio must divide 128");
+    // heads of 128: two query tiles a CTA (attention_wide_tc5.cu); its maxima are taken before the scale, which has to be positive
+    if (wide && d == 128 && scale > 0.f)
+        return telb_paged_attention_wide(q, kv_layer, out, q_start, q_len, past_len, page_table, tree_mask, mask_words, num_seqs, total_tokens,
+                                         num_pages, max_pages, page_size, hq, hkv, scale, window, splits, ws, ws_floats, is_bf16, status, stream);
     AttnParams p{};
     p.out = out;
     p.q_start = q_start;

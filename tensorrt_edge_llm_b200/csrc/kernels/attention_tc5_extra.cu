@@ -199,7 +199,7 @@ extern "C" int telb_paged_attention_dense(const void* q, const void* kv_layer, v
                                           const int* past_len, const int* page_table, const int* tree_mask, int mask_words,
                                           int num_seqs, int total_tokens, int max_q_len, int num_pages, int max_pages, int page_size,
                                           int hq, int hkv, int d, float scale, int window, int splits, float* ws, long long ws_floats,
-                                          int is_bf16, int* status, cudaStream_t stream);
+                                          int is_bf16, int* status, int wide, cudaStream_t stream);
 
 // Merge `splits` partial results (ws_o [splits, rows, d] fp32, ws_lse [splits, rows]) into out [rows, d].
 extern "C" int telb_attn_combine(const float* ws_o, const float* ws_lse, void* out, int rows, int splits, int d, int is_bf16,
@@ -237,14 +237,15 @@ extern "C" int telb_attn_combine_quant(const float* ws_o, const float* ws_lse, v
 }
 
 // q [T,Hq,D], kv_layer [pages,2,Hkv,P,D], out [T,Hq,D]; metadata as in the ragged step ABI.
-// ws must hold splits*T*Hq*(D+1) floats when splits > 1 (pass splits = 1 to avoid scratch).
+// ws must hold splits*T*Hq*(D+1) floats when splits > 1 (pass splits = 1 to avoid scratch).  wide: plain steps of head size 128 may
+// take the two-tile kernel.
 extern "C" int telb_paged_attention(const void* q, const void* kv_layer, void* out, const int* q_start,
                                     const int* q_len, const int* past_len, const int* page_table,
                                     const int* tree_mask, int mask_words, int num_seqs, int total_tokens,
                                     int max_q_len, int num_pages, int max_pages, int page_size, int hq, int hkv, int d,
                                     float scale, int window, int splits, float* ws, long long ws_floats, int is_bf16,
                                     int* status, const float* sinks, const float* skip_thr, int* skip_stats, int chunk, int split_p,
-                                    const float* back, float back_mult, const int* positions, long long ld_out, cudaStream_t stream) {
+                                    const float* back, float back_mult, const int* positions, long long ld_out, int wide, cudaStream_t stream) {
     if (num_seqs <= 0 || total_tokens <= 0) return 0;
     const int group = hkv > 0 ? hq / hkv : 0;
     if (!back && ld_out != (long long)hq * d) return fail("telb_paged_attention: rows further apart are built for rotated values");
@@ -252,7 +253,7 @@ extern "C" int telb_paged_attention(const void* q, const void* kv_layer, void* o
     if (sinks == nullptr && skip_thr == nullptr && chunk <= 0 && !split_p && !back && d != 256 && group > 0 && 128 % group == 0)
         return telb_paged_attention_dense(q, kv_layer, out, q_start, q_len, past_len, page_table, tree_mask, mask_words, num_seqs,
                                           total_tokens, max_q_len, num_pages, max_pages, page_size, hq, hkv, d, scale, window, splits,
-                                          ws, ws_floats, is_bf16, status, stream);
+                                          ws, ws_floats, is_bf16, status, wide, stream);
     if (d != 64 && d != 128 && d != 256) return fail("telb_paged_attention: head_dim must be 64, 128 or 256");
     if (page_size != 64 && page_size != 128) return fail("telb_paged_attention: page size must be 64 or 128");
     if (hkv <= 0 || hq % hkv) return fail("telb_paged_attention: Hq must be a multiple of Hkv");

@@ -606,6 +606,14 @@ def _attn_splits(meta: StepMeta, hkv: int, group: int, chunk: int = 0, window: i
     return max(1, min((2 * 148 + ctas - 1) // ctas, kv_tiles, 32))
 
 
+def _wide_splits(meta: StepMeta, hkv: int, group: int, window: int = 0) -> int:
+    """Splits of the two-tile kernel (head size 128): as many as fill the device, one CTA an SM, in one go, of at least 512 keys (a merge
+    of 300 rows cost more than the two thirds of 300 keys that it saved)."""
+    block = 2 * (128 // group)
+    blocks = min(meta.num_tokens // block + meta.num_seqs, meta.num_seqs * -(-meta.max_q_len // block))
+    return max(1, min(148 // max(1, blocks * hkv), _visible_len(meta, 0, window) // 512, 32))
+
+
 def _decode_splits(meta: StepMeta, hkv: int, chunk: int = 0, window: int = 0) -> int:
     ctas = meta.num_seqs * hkv
     if ctas >= 148:
@@ -619,10 +627,11 @@ def paged_attention(q, kv_layer, meta: StepMeta, scale, sliding_window=None, sin
                     skip_thr: Optional[torch.Tensor] = None, skip_stats: Optional[torch.Tensor] = None, chunk: int = 0,
                     fp32_weights: bool = False, back: Optional[tuple] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Paged GQA attention.  Decode-shaped steps (``max_q_len * Hq/Hkv <= 16``, head_dim 128, causal)
-    run the token-major XQA-style kernel; everything else the row-major tile kernel.
-    ``kernel`` forces ``"decode"`` or ``"tile"``; ``causal=False`` lets every row see every token of its sequence; ``chunk`` > 0 limits
+    run the token-major XQA-style kernel; everything else the row-major tile kernel, or its two-tile form for plain steps of head size 128.
+    ``kernel`` forces ``"decode"`` or ``"tile"`` (one tile a CTA); ``causal=False`` lets every row see every token of its sequence; ``chunk`` > 0 limits
     a row to the keys of its own ``chunk``-token block; ``fp32_weights`` feeds the probabilities to the 16-bit P·V product as high + low
     halves.  fp32 rows and head sizes without a tensor-core form run on the CUDA cores."""
+    wide = kernel is None
     if not causal:
         sliding_window, kernel = -1, "tile"
     if sinks is not None:
@@ -673,14 +682,15 @@ def paged_attention(q, kv_layer, meta: StepMeta, scale, sliding_window=None, sin
             "paged_attention_decode", 2 if splits > 1 else 1)
         return out
     if splits is None:
-        splits = _attn_splits(meta, hkv, group, chunk, win)
+        plain = wide and d == 128 and scale > 0 and sinks is None and skip_thr is None and chunk <= 0 and not fp32_weights and table is None and 128 % group == 0
+        splits = _wide_splits(meta, hkv, group, win) if plain else _attn_splits(meta, hkv, group, chunk, win)
     _check(lib().telb_paged_attention(
         _p(q), _p(kv_layer), _p(out), _p(meta.q_start), _p(meta.q_len), _p(meta.past_len), _p(meta.page_table),
         _p(tm), c_int(tm.shape[1] if tm is not None else 0), c_int(meta.num_seqs), c_int(t), c_int(meta.max_q_len),
         c_int(kv_layer.shape[0]), c_int(meta.page_table.shape[1]), c_int(meta.page_size), c_int(hq), c_int(hkv),
         c_int(d), c_float(scale), c_int(sliding_window or 0), c_int(splits), _p(ws.attn_ws), c_ll(ws.attn_ws.numel()),
         c_int(_is_bf16(q)), _p(ws.status), _p(sinks), _p(skip_thr), _p(skip_stats), c_int(chunk), c_int(int(fp32_weights)),
-        _p(table), c_float(mult), _p(meta.positions), c_ll(ld_out), _stream()), "paged_attention", 2 if splits > 1 else 1)
+        _p(table), c_float(mult), _p(meta.positions), c_ll(ld_out), c_int(int(wide)), _stream()), "paged_attention", 2 if splits > 1 else 1)
     return out
 
 

@@ -137,3 +137,54 @@ def test_recurrences_read_parts_of_wider_rows(cu, q_lens, pasts):
     y2 = cu.gated_delta_rule(q.contiguous(), k.contiguous(), v.contiguous(), a, b, A[:2], db[:2], st2, meta)
     assert torch.equal(y, y2) and torch.equal(st, st2)
     _check_status(cu)
+
+
+def _paged_step(q_lens, past_lens, hq, hkv, page, dtype, rows_masked=False):
+    from tensorrt_edge_llm_b200.ops import build_step_meta
+    g = torch.Generator(device="cuda").manual_seed(sum(q_lens) + hq)
+    n, most = len(q_lens), max((q + p + page - 1) // page for q, p in zip(q_lens, past_lens)) + 1
+    perm = torch.randperm(n * most + 3, generator=torch.Generator().manual_seed(hq))
+    table = torch.full((n, most), -1, dtype=torch.int32)
+    for i in range(n):
+        need = (q_lens[i] + past_lens[i] + page - 1) // page
+        table[i, :need] = perm[i * most:i * most + need].to(torch.int32)
+    kv = torch.randn(n * most + 3, 2, hkv, page, 128, device="cuda", generator=g).to(dtype)
+    q = torch.randn(sum(q_lens), hq, 128, device="cuda", generator=g).to(dtype)
+    more = {}
+    if rows_masked:
+        words = (max(q_lens) + 31) // 32
+        bits = torch.randint(-2 ** 31, 2 ** 31, (sum(q_lens), words), generator=torch.Generator().manual_seed(1))
+        r = 0
+        for ql in q_lens:
+            for i in range(ql):
+                bits[r, i // 32] |= (1 << (i % 32)) if i % 32 < 31 else -(1 << 31)       # every row sees itself
+                r += 1
+        more = dict(tree_mask=bits.to(torch.int32).cuda(), positions=torch.zeros(sum(q_lens), dtype=torch.int32), logits_all=True)
+    return q, kv, build_step_meta(q_lens, past_lens, table, page, device="cuda", **more)
+
+
+@pytest.mark.parametrize("q_lens,past_lens,hq,hkv,page,dtype", [
+    ([63, 64, 65], [0, 1, 127], 32, 8, 64, torch.bfloat16), ([1, 0, 129, 1], [300, 5, 64, 0], 8, 2, 64, torch.float16),
+    ([1] * 40 + [200], [70] * 40 + [3], 4, 1, 128, torch.bfloat16), ([257], [1000], 4, 4, 64, torch.bfloat16),
+    ([5, 40], [600, 2049], 16, 1, 128, torch.float16), ([3], [200], 128, 1, 64, torch.bfloat16)])
+def test_two_tile_attention(cu, q_lens, past_lens, hq, hkv, page, dtype):
+    """Blocks that end inside a tile, one-row sequences beside longer ones, key tiles across pages and past the end; causal, windowed,
+    unmasked; one split, several, and splits without a key."""
+    q, kv, meta = _paged_step(q_lens, past_lens, hq, hkv, page, dtype)
+    for kw in (dict(), dict(sliding_window=100), dict(causal=False)):
+        want = ref.paged_attention(q, kv, meta, 128 ** -0.5, **kw)
+        for splits in (1, 3, 7):
+            got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits, **kw)
+            # probabilities and outputs rounded to 16 bits (2^-8 each) over sums of weights of one sign
+            assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm(), (kw, splits)
+    _check_status(cu)
+
+
+@pytest.mark.parametrize("q_lens,past_lens", [([60, 60], [2048, 100]), ([16], [0]), ([33, 7, 64, 90], [63, 640, 65, 31])])
+def test_two_tile_attention_of_tree_rows(cu, q_lens, past_lens):
+    q, kv, meta = _paged_step(q_lens, past_lens, 32, 8, 64, torch.bfloat16, rows_masked=True)
+    want = ref.paged_attention(q, kv, meta, 128 ** -0.5)
+    for splits in (None, 1, 4):
+        got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits)
+        assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm(), splits
+    _check_status(cu)
