@@ -34,6 +34,7 @@
 // kernelSrcs/build_cutedsl.py:2164-2332; this kernel is written from the PTX up.
 #include "gemm_common.cuh"
 #include "nvfp4_common.cuh"
+#include "pair_common.cuh"
 
 namespace telb {
 
@@ -56,44 +57,6 @@ struct WideCfg {
     static constexpr int kSmem = kStages * kStage + 1024 + 256 + kRsStageBytes;
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank_w() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_w() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster.
-__device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(rank));
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
-// Shared-memory address of `ptr`'s counterpart in CTA `rank` of the cluster (shared::cluster window).
-__device__ __forceinline__ uint32_t cluster_addr_of(const void* ptr, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(ptr)), "r"(rank));
-    return remote;
-}
-// Tiled TMA load of a CTA pair (no multicast): the data lands in THIS CTA's shared memory, the byte count completes on the
-// mbarrier at `bar_cluster_addr`, which may belong to the other CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
-        : "memory");
-}
-// ---- cta_group::2 forms ------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc2(uint32_t* smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
 __device__ __forceinline__ void umma_nvfp4_2(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t tmem_sfa,
                                              uint32_t tmem_sfb, uint32_t accumulate) {
     asm volatile(
@@ -104,12 +67,6 @@ __device__ __forceinline__ void umma_nvfp4_2(uint32_t tmem_d, uint64_t desc_a, u
 __device__ __forceinline__ void tmem_cp_sf2(uint32_t tmem_dst, uint64_t desc_src) {
     asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc_src) : "memory");
 }
-// One arrive on `bar` in every CTA of `mask` once all MMAs issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit2(uint64_t* bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(mask) : "memory");
-}
-
 struct WideTile {
     int a0, b0, tb;        // first row of the (pair) tile, first column, column-tile index
 };
@@ -426,53 +383,11 @@ static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
                        const GemmParams& p, cudaStream_t stream) {
     using Cfg = WideCfg;
     auto kern = gemm_nvfp4_wide_kernel;
-    static int max_clusters = 0;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
-        if (e != cudaSuccess) return fail("cudaFuncSetAttribute(gemm_nvfp4_wide)", e);
-        // how many pairs can be resident at once: a pair needs two free SMs of one TPC / GPC, so it is queried, not assumed
-        cudaLaunchConfig_t q{};
-        q.gridDim = dim3(sm_count() / 2 * 2, 1, 1);
-        q.blockDim = dim3(kGemmThreads, 1, 1);
-        q.dynamicSmemBytes = Cfg::kSmem;
-        cudaLaunchAttribute a[1];
-        a[0].id = cudaLaunchAttributeClusterDimension;
-        a[0].val.clusterDim.x = 2;
-        a[0].val.clusterDim.y = 1;
-        a[0].val.clusterDim.z = 1;
-        q.attrs = a;
-        q.numAttrs = 1;
-        int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, kern, &q);
-        if (e != cudaSuccess || n <= 0) {
-            cudaGetLastError();
-            n = sm_count() / 2;
-        }
-        max_clusters = n;
-        if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", n, sm_count());
-        configured = true;
-    }
+    static const int max_pairs = resident_pairs(kern, kGemmThreads, Cfg::kSmem);
+    if (max_pairs <= 0) return fail("gemm_nvfp4_wide: configuration");
+    if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", max_pairs, sm_count());
     const int total = p.tiles_a * p.tiles_b;
-    const int clusters = total < max_clusters ? total : max_clusters;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(clusters * 2, 1, 1);
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::kSmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attrs[2];
-    int na = 0;
-    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[na].val.programmaticStreamSerializationAllowed = 1;
-    if (pdl_enabled()) ++na;
-    attrs[na].id = cudaLaunchAttributeClusterDimension;
-    attrs[na].val.clusterDim.x = 2;
-    attrs[na].val.clusterDim.y = 1;
-    attrs[na].val.clusterDim.z = 1;
-    ++na;
-    cfg.attrs = attrs;
-    cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tsfa, tsfb, k64, k64, p);
+    const cudaError_t e = launch_pairs(kern, total < max_pairs ? total : max_pairs, kGemmThreads, Cfg::kSmem, stream, ta, tb, tsfa, tsfb, k64, k64, p);
     if (e != cudaSuccess) return fail("cudaLaunchKernelEx(gemm_nvfp4_wide)", e);
     return 0;
 }

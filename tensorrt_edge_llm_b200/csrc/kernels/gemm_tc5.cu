@@ -186,12 +186,16 @@ extern "C" int telb_gemm_skinny_fused(int kind, const void* x, const void* x_sf,
 extern "C" int telb_gemm_skinny_f32out(const void* x, const void* w, float* out, int M, int N, int K, const float* bias, int is_bf16,
                                        int* status, cudaStream_t stream);
 
+extern "C" int telb_gemm_pair_pays(int M, int N);
+extern "C" int telb_gemm_pair(const void* x, const void* w, void* out, int M, int N, int K, const void* bias, const float* alpha,
+                              const void* residual, int epi, int is_bf16, int* status, cudaStream_t stream);
+
 extern "C" const char* telb_last_error() { return g_last_error; }
 
 // out[M,N] = x[M,K] · w[N,K]^T  (16-bit row-major operands, K % 8 == 0).
 //   bias / alpha : per output column (may be null);  residual : [M,N] like out (may be null)
 //   ws / counters: split-K scratch, used only by the small-M path (ws_bytes may be 0 → no split)
-//   mode         : 0 = choose, 1 = force large-M layout, 2 = force swapped layout
+//   mode         : 0 = choose (prompt sizes: also the CTA-pair kernel, gemm_pair_tc5.cu), 1 = force large-M layout, 2 = force swapped layout
 static int gemm_f16_impl(const void* x, const void* w, void* out, int M, int N, int K, const void* bias,
                          const float* alpha, const void* residual, int is_bf16, void* ws, long long ws_bytes,
                          int* counters, int n_counters, int* status, int mode, int force_splits,
@@ -208,6 +212,8 @@ static int gemm_f16_impl(const void* x, const void* w, void* out, int M, int N, 
         return telb_gemm_skinny_f32out(x, w, (float*)out, M, N, K, (const float*)bias, is_bf16, status, stream);
     if (mode == 0 && M <= 128)
         return telb_gemm_skinny(0, x, nullptr, w, nullptr, out, M, N, K, alpha, bias, residual, is_bf16, status, 0, stream);
+    if (mode == 0 && !out_f32 && telb_gemm_pair_pays(M, N))
+        return telb_gemm_pair(x, w, out, M, N, K, bias, alpha, residual, 0, is_bf16, status, stream);
     const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const bool swapped = mode == 2 || (mode == 0 && M <= 128);
     GemmParams p{};

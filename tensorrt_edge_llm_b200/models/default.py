@@ -23,7 +23,7 @@ from .. import ops
 from ..config import ModelConfig
 from ..ops.meta import StepMeta
 from ..parallel.comm import LocalComm
-from .linear import HeadLinear, NVFP4Linear, SplitHeadLinear, TPMode, make_linear
+from .linear import HeadLinear, Linear, NVFP4Linear, SplitHeadLinear, TPMode, make_linear
 
 
 class RMSNorm(nn.Module):
@@ -373,9 +373,13 @@ class MLP(nn.Module):
                 if not isinstance(x, torch.Tensor) and (rows > 128 or small):
                     return self.down_proj(gp.forward_swiglu(x, scale))
                 return self.down_proj(ops.swiglu(gp(x), scale, interleaved=True))
+        gated, scale = self.act in ("silu", "swiglu"), self.down_proj.fused_input_scale()
+        # plain 16-bit rows and weights (no adapter, collective or bias between product and activation)
+        if (type(gp) is Linear and scale is None and gp.bias is None and gp.rs_comm is None and isinstance(x, torch.Tensor) and x.dim() == 2
+                and getattr(x, "ag_wait", None) is None):
+            return self.down_proj(ops.linear_act(x, gp.weight, "swiglu" if gated else "relu2"))
         gu = gp(x)
-        a = ops.swiglu(gu, self.down_proj.fused_input_scale()) if self.act in ("silu", "swiglu") else ops.relu2(gu)
-        return self.down_proj(a)
+        return self.down_proj(ops.swiglu(gu, scale) if gated else ops.relu2(gu))
 
 
 class DecoderLayer(nn.Module):

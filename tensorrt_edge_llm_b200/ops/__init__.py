@@ -137,6 +137,14 @@ def embedding(ids, table):
     return ref.embedding(ids, table)
 
 
+def linear_act(x, weight, act):
+    """``swiglu`` (gate rows of ``weight`` first) or ``relu2`` of ``x · weightᵀ``."""
+    if x.is_cuda:
+        return cuda_ops().gemm_act(x, weight, act)
+    y = linear(x, weight)
+    return swiglu(y) if act == "swiglu" else relu2(y)
+
+
 def linear(x, weight, bias=None):
     if x.is_cuda:
         return cuda_ops().gemm(x, weight, bias)

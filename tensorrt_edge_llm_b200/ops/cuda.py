@@ -319,6 +319,21 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = N
     return out.reshape(*lead, n)
 
 
+def gemm_act(x: torch.Tensor, weight: torch.Tensor, act: str) -> torch.Tensor:
+    """``relu2`` of ``x · weightᵀ``, or ``swiglu`` of it (gate rows of ``weight`` first): in the product's epilogue where the pair kernel
+    is the one to take, else as a pass of its own.  The same bits either way."""
+    m, k = x.shape
+    n, rows = weight.shape[0] // (2 if act == "swiglu" else 1), weight.shape[0]
+    if not (k % 8 == 0 and n % 8 == 0 and weight.dtype == x.dtype and x.dtype != torch.float32 and x.is_contiguous() and weight.is_contiguous()
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and lib().telb_gemm_pair_pays(c_int(m), c_int(rows))):
+        y = gemm(x, weight)
+        return swiglu(y) if act == "swiglu" else relu2(y)
+    out = torch.empty(m, n, dtype=x.dtype, device=x.device)
+    _check(lib().telb_gemm_pair(_p(x), _p(weight), _p(out), c_int(m), c_int(n), c_int(k), _p(None), _p(None), _p(None),
+                                c_int(1 if act == "swiglu" else 2), c_int(_is_bf16(x)), _p(Workspace.get(x.device).status), _stream()), "gemm_pair")
+    return out
+
+
 def gemm_f32out(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[M,N]`` fp32 ``= x · weightᵀ (+ bias)``: tensor-core product of 16-bit operands, or the fp32 kernel for fp32 operands.
     ``bias`` is fp32."""

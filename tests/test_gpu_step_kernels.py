@@ -188,3 +188,31 @@ def test_two_tile_attention_of_tree_rows(cu, q_lens, past_lens):
         got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits)
         assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm(), splits
     _check_status(cu)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(129, 264, 8), (256, 512, 64), (257, 1040, 136), (700, 3000, 200), (5000, 2064, 520)])
+def test_pair_gemm_equals_the_single_cta_kernel(cu, m, n, k, dtype):
+    """256 x 256 tiles: ragged rows, columns and K steps, more tiles than pairs; bias, scale and residual; SwiGLU and squared ReLU in the
+    epilogue.  Both kernels add the same products in the same order."""
+    from tensorrt_edge_llm_b200.ops.cuda import _check, _p, _stream, c_int
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x, w = torch.randn(m, k, device="cuda", generator=g).to(dtype), torch.randn(n, k, device="cuda", generator=g).to(dtype)
+    bias, res = torch.randn(n, device="cuda", generator=g).to(dtype), torch.randn(m, n, device="cuda", generator=g).to(dtype)
+    alpha = torch.rand(n, device="cuda", generator=g)
+
+    def pair(cols, epi, b=None, a=None, r=None):
+        out = torch.full((m, cols), float("nan"), device="cuda", dtype=dtype)
+        _check(cu.lib().telb_gemm_pair(_p(x), _p(w), _p(out), c_int(m), c_int(cols), c_int(k), _p(b), _p(a), _p(r), c_int(epi),
+                                       c_int(int(dtype == torch.bfloat16)), _p(cu.Workspace.get(x.device).status), _stream()), "gemm_pair")
+        return out
+
+    plain = cu.gemm(x, w, mode=1)
+    assert torch.equal(pair(n, 0), plain)
+    assert torch.equal(pair(n, 0, bias, alpha, res), cu.gemm(x, w, bias, alpha, res, mode=1))
+    assert torch.equal(pair(n // 2, 1), cu.swiglu(plain)) if n % 16 == 0 else True
+    assert torch.equal(pair(n, 2), cu.relu2(plain))
+    for act in ("swiglu", "relu2"):
+        if act == "relu2" or n % 16 == 0:
+            assert torch.equal(cu.gemm_act(x, w, act), getattr(cu, act)(plain))
+    _check_status(cu)
