@@ -81,34 +81,50 @@ def build_step_meta(q_lens: Sequence[int], past_lens: Sequence[int], page_table:
     """Host-side construction of a :class:`StepMeta` (the Python twin of the native builder).  Logits are computed for the last row of
     every sequence, for all rows (``logits_all``) or for the listed packed rows (``logits_rows``)."""
     n = len(q_lens)
-    q_start = [0]
-    for q in q_lens:
-        q_start.append(q_start[-1] + int(q))
-    t = q_start[-1]
-    pos: List[int] = []
-    sid: List[int] = []
-    for i, (q, p) in enumerate(zip(q_lens, past_lens)):
-        pos.extend(range(int(p), int(p) + int(q)))
-        sid.extend([i] * int(q))
+    q_lens, past_lens = [int(q) for q in q_lens], [int(p) for p in past_lens]
+    i32 = dict(dtype=torch.int32)
+    q, past = torch.tensor(q_lens, **i32), torch.tensor(past_lens, **i32)
+    q_start = torch.zeros(n + 1, **i32)
+    torch.cumsum(q, 0, out=q_start[1:])
+    t = int(q_start[n])
+    sid = torch.repeat_interleave(torch.arange(n, **i32), q)
     pos_t = None
     if isinstance(positions, torch.Tensor):          # already on the device (tree steps): no host copy of the values
         pos_t = positions.to(device=device, dtype=torch.int32).reshape(-1)
+        pos = torch.zeros(0, **i32)
     elif positions is not None:
-        pos = [int(x) for x in positions]
-    if logits_rows is not None:
-        lidx = [int(r) for r in logits_rows]
-    elif logits_all:
-        lidx = list(range(t))
+        pos = torch.tensor([int(x) for x in positions], **i32)
     else:
-        lidx = [q_start[i + 1] - 1 for i in range(n)]
-    i32 = dict(dtype=torch.int32, device=device)
+        pos = torch.arange(t, **i32) + torch.repeat_interleave(past - q_start[:n], q)
+    if logits_rows is not None:
+        lidx = torch.tensor([int(r) for r in logits_rows], **i32)
+    elif logits_all:
+        lidx = torch.arange(t, **i32)
+    else:
+        lidx = q_start[1:] - 1
+    slots = torch.tensor([int(x) for x in slot_ids] if slot_ids is not None else list(range(n)), **i32)
+    parts = [q_start, q, past, pos, sid, slots, lidx]
+    table = page_table.to(**i32)
+    if table.device.type == "cpu":
+        parts.append(table)
+    parts = _upload(parts, device)
+    q_start, q, past, pos, sid, slots, lidx = parts[:7]
+    table = parts[7] if len(parts) > 7 else table.to(device)
     return StepMeta(
-        q_start=torch.tensor(q_start, **i32), q_len=torch.tensor(list(q_lens), **i32),
-        past_len=torch.tensor(list(past_lens), **i32), positions=pos_t if pos_t is not None else torch.tensor(pos, **i32),
-        seq_ids=torch.tensor(sid, **i32), page_table=page_table.to(device=device, dtype=torch.int32),
-        slot_ids=torch.tensor(list(slot_ids) if slot_ids is not None else list(range(n)), **i32),
-        logits_idx=torch.tensor(lidx, **i32), page_size=page_size, num_seqs=n, num_tokens=t,
-        max_q_len=max(q_lens) if n else 0,
-        max_seq_len=max((int(q) + int(p) for q, p in zip(q_lens, past_lens)), default=0),
-        tree_mask=tree_mask.to(device) if tree_mask is not None else None,
-        host_lens=tuple((int(q), int(p)) for q, p in zip(q_lens, past_lens)))
+        q_start=q_start, q_len=q, past_len=past, positions=pos_t if pos_t is not None else pos, seq_ids=sid, page_table=table, slot_ids=slots,
+        logits_idx=lidx, page_size=page_size, num_seqs=n, num_tokens=t, max_q_len=max(q_lens) if n else 0,
+        max_seq_len=max((q + p for q, p in zip(q_lens, past_lens)), default=0),
+        tree_mask=tree_mask.to(device) if tree_mask is not None else None, host_lens=tuple(zip(q_lens, past_lens)))
+
+
+def _upload(parts: List[torch.Tensor], device) -> List[torch.Tensor]:
+    """int32 host tensors on ``device``.  To a GPU they travel as one copy from pinned memory that the host does not wait for: a blocking
+    copy per tensor made it wait for the step before and left the GPU idle while this one was put together (0.5 ms of a 3.4 ms step)."""
+    if torch.device(device).type != "cuda":
+        return [p.to(device) for p in parts]
+    sizes = [(p.numel() + 31) // 32 * 32 for p in parts]           # every part starts on 128 bytes
+    host = torch.zeros(sum(sizes), dtype=torch.int32, pin_memory=True)
+    for p, h in zip(parts, host.split(sizes)):
+        h[:p.numel()].copy_(p.reshape(-1))
+    dev = host.to(device, non_blocking=True)
+    return [d[:p.numel()].view(p.shape) for p, d in zip(parts, dev.split(sizes))]
