@@ -449,14 +449,18 @@ extern "C" int telb_gemm_nvfp4_swiglu(const void* xq, const void* x_sf, const vo
 
 // Grouped NVFP4 GEMM for mixture-of-experts (see telb_gemm_f16_grouped): xq [rows_pad, K/2] with
 // atom-layout scales over the padded row space, wq [experts * N, K/2] with scales over experts * N rows.
+extern "C" int telb_gemm_nvfp4_tile_grouped_launch(const void* xq, const void* x_sf, const void* wq, const void* w_sf, int rows_pad, int K, int experts,
+                                                   const void* params_blob, cudaStream_t stream);
+constexpr long long kGroupedTileMin = 148;
+
 static int gemm_nvfp4_grouped_impl(const void* xq, const void* x_sf, const void* wq, const void* w_sf, void* out, int rows_pad, int N, int K,
                                    int experts, const int* tile_expert, const float* alpha, int out_bf16, int* status, cudaStream_t stream,
-                                   const SwigluOut* sw);
+                                   const SwigluOut* sw, int slots);
 
 extern "C" int telb_gemm_nvfp4_grouped(const void* xq, const void* x_sf, const void* wq, const void* w_sf, void* out,
                                        int rows_pad, int N, int K, int experts, const int* tile_expert, const float* alpha,
-                                       int out_bf16, int* status, cudaStream_t stream) {
-    return gemm_nvfp4_grouped_impl(xq, x_sf, wq, w_sf, out, rows_pad, N, K, experts, tile_expert, alpha, out_bf16, status, stream, nullptr);
+                                       int out_bf16, int* status, int slots, cudaStream_t stream) {
+    return gemm_nvfp4_grouped_impl(xq, x_sf, wq, w_sf, out, rows_pad, N, K, experts, tile_expert, alpha, out_bf16, status, stream, nullptr, slots);
 }
 
 // Grouped gate/up projection with SwiGLU and the NVFP4 quantisation of the second expert GEMM's input in the epilogue.
@@ -470,12 +474,20 @@ extern "C" int telb_gemm_nvfp4_grouped_swiglu(const void* xq, const void* x_sf, 
     if (N % 128) return fail("telb_gemm_nvfp4_grouped_swiglu: 2 * inter must be a multiple of 128");
     if (!out_xq || !out_sf || !out_global_scale) return fail("telb_gemm_nvfp4_grouped_swiglu: output buffers and scale are required");
     SwigluOut sw{static_cast<uint8_t*>(out_xq), static_cast<uint8_t*>(out_sf), out_global_scale, N / 4, telb_nvfp4_k64_pad(N / 2)};
-    return gemm_nvfp4_grouped_impl(xq, x_sf, wq, w_sf, nullptr, rows_pad, N, K, experts, tile_expert, alpha, out_bf16, status, stream, &sw);
+    return gemm_nvfp4_grouped_impl(xq, x_sf, wq, w_sf, nullptr, rows_pad, N, K, experts, tile_expert, alpha, out_bf16, status, stream, &sw, 0);
+}
+
+// Whether the grouped product takes 128 x 256 tiles.  `slots`: routed rows (0: unknown), of which at most one per expert opens a row tile
+// of its own.  From about a wave of wide tiles on they are the faster ones (128 experts of 1536 x 2048 and 2048 x 768, mean of both products:
+// 4 tokens of 8 experts 21.0 -> 15.3 us, 32: 48 -> 32, 1024: 58 -> 46, 8000: 222 -> 138); below, twice as many narrow tiles fill more SMs.
+static bool grouped_takes_tile(int slots, int rows_pad, int experts, int N) {
+    const long long row_tiles = slots > 0 ? slots / kBM + (slots < experts ? slots : experts) : rows_pad / kBM;
+    return row_tiles * ((N + 255) / 256) >= kGroupedTileMin;
 }
 
 static int gemm_nvfp4_grouped_impl(const void* xq, const void* x_sf, const void* wq, const void* w_sf, void* out, int rows_pad, int N, int K,
                                    int experts, const int* tile_expert, const float* alpha, int out_bf16, int* status, cudaStream_t stream,
-                                   const SwigluOut* sw) {
+                                   const SwigluOut* sw, int slots) {
     if (rows_pad <= 0) return 0;
     if (K % 32 || rows_pad % kBM || N % 128) return fail("telb_gemm_nvfp4_grouped: K % 32, rows_pad % 128 and N % 128 must be 0");
     GemmParams p{};
@@ -498,6 +510,8 @@ static int gemm_nvfp4_grouped_impl(const void* xq, const void* x_sf, const void*
         p.sw_ld = sw->ld;
         p.sw_k64_pad = sw->k64_pad;
     }
+    if (telb_nvfp4_wide_mode() == 1 && grouped_takes_tile(slots, rows_pad, experts, N))
+        return telb_gemm_nvfp4_tile_grouped_launch(xq, x_sf, wq, w_sf, rows_pad, K, experts, &p, stream);
     const uint64_t kbytes = (uint64_t)K / 2;
     CUtensorMap ta, tb;
     if (make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, rows_pad, kbytes, kbytes, kBM, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;

@@ -14,6 +14,10 @@
 // Roles (14 warps): 0 TMA producer, 1 MMA issuer / TMEM owner, 2-9 epilogue (two warps per lane quadrant, 64 columns of a half each),
 // 10-13 scale factors.  Every wait is bounded.
 //
+// Grouped form (mixture of experts): a row tile belongs to one expert, `tile_expert` names its weight block and how many of its rows are in
+// use.  Tiles of few rows (a decode step routes two or three tokens to an expert) load 32 rows of x instead of 128.  Their K loops are
+// short (3 to 8 steps), so the column scales are fetched to shared memory while the MMAs run.
+//
 // RS: the reduce-scatter form stages rows in shared memory so that they leave as 128-byte lines to their owner rank, in the place of
 // the fourth operand stage.  No TMA load here uses cluster multicast (the kernel runs inside tensor-parallel steps too).
 #include "gemm_common.cuh"
@@ -36,11 +40,13 @@ struct NtCfg {
     static constexpr int kStage = kATile + kBTile + kSf;
     static constexpr int kStages = RS ? 3 : 4;
     static constexpr int kSlab = RS ? kNtEpiWarps * 32 * kRsStageRowBytes : 0;
-    static constexpr int kSmem = kStages * kStage + 1024 + 256 + kSlab;
+    static constexpr int kSmem = kStages * kStage + 1024 + 256 + kSlab + (RS ? 0 : kNtEpiWarps * 128 * 4);
 };
 
 struct NtTile {
     int a0, b0, tb;
+    int brow;              // first weight row of the tile's expert (0: one weight for all rows)
+    int rows;              // rows of the tile in use; 0 = nothing to do
 };
 __device__ __forceinline__ NtTile nt_tile(const GemmParams& p, int t) {
     const int per_group = kRasterGroup * p.tiles_b;
@@ -52,6 +58,13 @@ __device__ __forceinline__ NtTile nt_tile(const GemmParams& p, int t) {
     w.a0 = (gfirst + within % gsize) * kBM;
     w.tb = within / gsize;
     w.b0 = w.tb * kNtBN;
+    w.brow = 0;
+    w.rows = 128;
+    if (p.tile_expert) {
+        const int ta = w.a0 / kBM, e = p.tile_expert[ta];
+        w.rows = e < 0 ? 0 : p.tile_expert[p.tiles_a + ta];
+        w.brow = max(e, 0) * p.group_rows_b;
+    }
     return w;
 }
 
@@ -63,7 +76,7 @@ __device__ __forceinline__ void st_global_32b(void* dst, const uint4& a, const u
 // 32 gate and 32 up sums of one row → 32 quantised SwiGLU outputs (features f0 .. f0 + 31): the same roundings as the unfused
 // chain (16-bit GEMM output, 16-bit activation), then quantise.
 template <typename T>
-__device__ __forceinline__ void nt_swiglu(const GemmParams& p, const uint32_t (&rg)[32], const uint32_t (&ru)[32], int row, int gcol, int ucol, int f0,
+__device__ __forceinline__ void nt_swiglu(const GemmParams& p, const uint32_t (&rg)[32], const uint32_t (&ru)[32], int row, const float* ga, const float* ua, int f0,
                                           float gs, float inv_gs) {
     uint2 packed[2];
     uint8_t s8[2];
@@ -75,9 +88,9 @@ __device__ __forceinline__ void nt_swiglu(const GemmParams& p, const uint32_t (&
         for (int k = 0; k < 16; ++k) {
             const int j = hf * 16 + k;
             float g = __uint_as_float(rg[j]), u = __uint_as_float(ru[j]);
-            if (p.alpha) {
-                g *= __ldg(&p.alpha[gcol + j]);
-                u *= __ldg(&p.alpha[ucol + j]);
+            if (ga) {
+                g *= ga[j];
+                u *= ua[j];
             }
             g = Cvt<T>::to_f(Cvt<T>::from_f(g));
             u = Cvt<T>::to_f(Cvt<T>::from_f(u));
@@ -119,7 +132,8 @@ __device__ __forceinline__ void nt_store32(const GemmParams& p, const uint32_t (
 
 template <bool RS>
 __global__ void __launch_bounds__(kNtThreads, 1)
-gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const uint8_t* __restrict__ sf_a,
+gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a32,
+                       const __grid_constant__ CUtensorMap tma_b, const uint8_t* __restrict__ sf_a,
                        const uint8_t* __restrict__ sf_b, int sf_k64, GemmParams p) {
     using Cfg = NtCfg<RS>;
     constexpr int STAGES = Cfg::kStages;
@@ -136,6 +150,7 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tovl_bar + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     uint8_t* slab0 = smem + STAGES * Cfg::kStage + 256;
+    float* s_alpha = reinterpret_cast<float*>(slab0);      // column scales of the tile, 128 per epilogue warp (grouped form, which has no slab)
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -179,10 +194,13 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
             const int last_a = (p.rows_a - 1) / 128, last_b = (p.rows_b - 1) / 128;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 const NtTile w = nt_tile(p, t);
+                if (w.rows == 0) continue;
+                const bool few = w.rows <= 32;
+                const int eb = w.brow / 128;
                 if (p.ag_flags && !ag_wait_rows(p, w.a0, ag_e, abort_flag)) break;
                 const uint8_t* ga = sf_a + (size_t)min(w.a0 / 128, last_a) * sf_k64 * 512;
-                const uint8_t* gb0 = sf_b + (size_t)min(w.b0 / 128, last_b) * sf_k64 * 512;
-                const uint8_t* gb1 = sf_b + (size_t)min(w.b0 / 128 + 1, last_b) * sf_k64 * 512;
+                const uint8_t* gb0 = sf_b + (size_t)(eb + min(w.b0 / 128, last_b)) * sf_k64 * 512;
+                const uint8_t* gb1 = sf_b + (size_t)(eb + min(w.b0 / 128 + 1, last_b)) * sf_k64 * 512;
                 for (int kb = 0; kb < p.kb_total; ++kb) {
                     if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kStatusProducerTimeout)) {
                         ok = false;
@@ -195,9 +213,9 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     bulk_load(ss, ga + (size_t)kb * 2048, 2048, &sfull_bar[stage]);
                     bulk_load(ss + 2048, gb0 + (size_t)kb * 2048, 2048, &sfull_bar[stage]);
                     bulk_load(ss + 4096, gb1 + (size_t)kb * 2048, 2048, &sfull_bar[stage]);
-                    mbar_expect_tx(&full_bar[stage], Cfg::kATile + Cfg::kBTile);
-                    tma_load_2d(sa, &tma_a, &full_bar[stage], kb * 128, w.a0);
-                    tma_load_2d(sb, &tma_b, &full_bar[stage], kb * 128, w.b0);
+                    mbar_expect_tx(&full_bar[stage], (few ? Cfg::kATile / 4 : Cfg::kATile) + Cfg::kBTile);
+                    tma_load_2d(sa, few ? &tma_a32 : &tma_a, &full_bar[stage], kb * 128, w.a0);      // few: the other rows keep what was there
+                    tma_load_2d(sb, &tma_b, &full_bar[stage], kb * 128, w.brow + w.b0);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -212,8 +230,10 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
             int stage = 0;
             uint32_t phase = 0, buf = 0, bphase = 0;
             bool ok = true;
-            int i = 0;
-            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++i) {
+            int i = -1;
+            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+                if (nt_tile(p, t).rows == 0) continue;
+                ++i;
                 const int acc = i & 1;
                 const uint32_t use_par = (uint32_t)(i >> 1) & 1u;
                 // the accumulator's previous tile is fully drained, and the previous tile's overlapping half is drained
@@ -254,6 +274,7 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kNtSf0;
         bool ok = true;
         for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+            if (nt_tile(p, t).rows == 0) continue;
             for (int kb = 0; kb < p.kb_total; ++kb) {
                 if (!mbar_wait(&sfull_bar[stage], phase, abort_flag, p.status, kStatusMmaTimeout)) {
                     ok = false;
@@ -293,23 +314,40 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
         // ---------------- epilogue: lane quadrant `quad`, column group `grp` of every half ----------------
         const int quad = warp & 3, grp = (warp - 2) >> 2;
         const bool wide_rows = !p.residual && p.rows_b % 16 == 0 && (reinterpret_cast<uintptr_t>(p.c) & 31) == 0;
-        int i = 0;
-        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++i) {
+        int i = -1;
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
             const NtTile w = nt_tile(p, t);
+            if (w.rows == 0) continue;
+            ++i;
             const int acc = i & 1;
+            const bool sw = p.sw_xq != nullptr;
+            // SwiGLU: columns [0,64) of a half are gate features, [64,128) the matching up features; 32 of each per warp
+            const int c0 = sw ? grp * 32 : grp * 64, c1 = sw ? 64 + grp * 32 : grp * 64 + 32;
+            const float* buf = nullptr;
+            if (!RS && p.tile_expert && p.alpha) {
+                float* own = s_alpha + (warp - 2) * 128;
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int col = w.b0 + (q >> 1) * 128 + ((q & 1) ? c1 : c0) + lane;
+                    own[q * 32 + lane] = col < p.rows_b ? __ldg(&p.alpha[w.brow + col]) : 0.f;
+                }
+                __syncwarp();
+                buf = own;
+            }
             if (!mbar_wait(&tfull_bar[acc], (uint32_t)(i >> 1) & 1u, abort_flag, p.status, kStatusEpilogueTimeout)) break;
             tc_fence_after_sync();
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (acc ? kNtAcc1 : 0);
             const int row = w.a0 + quad * 32 + lane;
-            const bool row_ok = row < p.rows_a;
+            const bool row_ok = row < p.rows_a && quad * 32 + lane < w.rows;
 #pragma unroll 1
             for (int hh = 0; hh < 2; ++hh) {
                 // accumulator 0 gives up its upper half first (accumulator 1 begins there), accumulator 1 its lower half
                 const int h = acc ? hh : (hh ^ 1);
                 const int hb0 = w.b0 + h * 128;
-                const bool sw = p.sw_xq != nullptr;
-                // SwiGLU: columns [0,64) of the half are gate features, [64,128) the matching up features; 32 of each per warp
-                const int c0 = sw ? grp * 32 : grp * 64, c1 = sw ? 64 + grp * 32 : grp * 64 + 32;
+                // scales of the two 32-column pieces of this half
+                const float* a0 = buf ? buf + h * 64 : p.alpha ? p.alpha + hb0 + c0 : nullptr;
+                const float* a1 = buf ? buf + h * 64 + 32 : p.alpha ? p.alpha + hb0 + c1 : nullptr;
                 uint32_t r0[32], r1[32];
                 tmem_ld_x32(t_addr + h * 128 + c0, r0);
                 tmem_ld_x32(t_addr + h * 128 + c1, r1);
@@ -321,8 +359,8 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     if (row_ok && hb0 + 128 <= p.rows_b) {
                         const float gs = *p.sw_gs;
                         const int f0 = (w.tb * 2 + h) * 64 + grp * 32;
-                        if (p.out_bf16) nt_swiglu<__nv_bfloat16>(p, r0, r1, row, hb0 + c0, hb0 + c1, f0, gs, 1.f / gs);
-                        else nt_swiglu<__half>(p, r0, r1, row, hb0 + c0, hb0 + c1, f0, gs, 1.f / gs);
+                        if (p.out_bf16) nt_swiglu<__nv_bfloat16>(p, r0, r1, row, a0, a1, f0, gs, 1.f / gs);
+                        else nt_swiglu<__half>(p, r0, r1, row, a0, a1, f0, gs, 1.f / gs);
                     }
                 } else if (RS) {
                     uint8_t* slab = slab0 + (warp - 2) * (32 * kRsStageRowBytes);
@@ -356,12 +394,17 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
                     }
                     __syncwarp();
                 } else if (row_ok) {
+                    GemmParams p0 = p, p1 = p;
+                    if (buf) {
+                        p0.alpha = a0 - (hb0 + c0);
+                        p1.alpha = a1 - (hb0 + c1);
+                    }
                     if (p.out_bf16) {
-                        nt_store32<__nv_bfloat16>(p, r0, row, hb0 + c0, wide_rows);
-                        nt_store32<__nv_bfloat16>(p, r1, row, hb0 + c1, wide_rows);
+                        nt_store32<__nv_bfloat16>(p0, r0, row, hb0 + c0, wide_rows);
+                        nt_store32<__nv_bfloat16>(p1, r1, row, hb0 + c1, wide_rows);
                     } else {
-                        nt_store32<__half>(p, r0, row, hb0 + c0, wide_rows);
-                        nt_store32<__half>(p, r1, row, hb0 + c1, wide_rows);
+                        nt_store32<__half>(p0, r0, row, hb0 + c0, wide_rows);
+                        nt_store32<__half>(p1, r1, row, hb0 + c1, wide_rows);
                     }
                 }
             }
@@ -384,7 +427,7 @@ gemm_nvfp4_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
 }
 
 template <bool RS>
-static int launch_tile(const CUtensorMap& ta, const CUtensorMap& tb, const uint8_t* sfa, const uint8_t* sfb, int k64, const GemmParams& p,
+static int launch_tile(const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& tb, const uint8_t* sfa, const uint8_t* sfb, int k64, const GemmParams& p,
                        cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
@@ -394,7 +437,7 @@ static int launch_tile(const CUtensorMap& ta, const CUtensorMap& tb, const uint8
     }
     const int total = p.tiles_a * p.tiles_b;
     const int grid = total < sm_count() ? total : sm_count();
-    TELB_LAUNCH("gemm_nvfp4_tile_kernel", (gemm_nvfp4_tile_kernel<RS>), dim3(grid), dim3(kNtThreads), NtCfg<RS>::kSmem, stream, ta, tb, sfa, sfb, k64, p);
+    TELB_LAUNCH("gemm_nvfp4_tile_kernel", (gemm_nvfp4_tile_kernel<RS>), dim3(grid), dim3(kNtThreads), NtCfg<RS>::kSmem, stream, ta, ta32, tb, sfa, sfb, k64, p);
     TELB_CHECK_LAUNCH("gemm_nvfp4_tile_kernel");
     return 0;
 }
@@ -426,6 +469,21 @@ extern "C" int telb_gemm_nvfp4_tile_launch(const void* xq, const void* x_sf, con
     if (make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, M, kbytes, kbytes, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     if (make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, N, kbytes, kbytes, 256, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     const int k64 = p.kb_total * 4;
-    return p.rs_world > 1 ? launch_tile<true>(ta, tb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, p, stream)
-                          : launch_tile<false>(ta, tb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, p, stream);
+    return p.rs_world > 1 ? launch_tile<true>(ta, ta, tb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, p, stream)
+                          : launch_tile<false>(ta, ta, tb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, k64, p, stream);
+}
+
+// Grouped form: `params_blob` carries the epilogue fields, tile_expert and the weight rows per expert (rows_b = group_rows_b = N).
+extern "C" int telb_gemm_nvfp4_tile_grouped_launch(const void* xq, const void* x_sf, const void* wq, const void* w_sf, int rows_pad, int K, int experts,
+                                                   const void* params_blob, cudaStream_t stream) {
+    GemmParams p = *static_cast<const GemmParams*>(params_blob);
+    const uint64_t kbytes = (uint64_t)K / 2;
+    p.kb_total = (K + 255) / 256;
+    p.tiles_a = rows_pad / kBM;
+    p.tiles_b = (p.rows_b + kNtBN - 1) / kNtBN;
+    CUtensorMap ta, ta32, tb;
+    if (make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, rows_pad, kbytes, kbytes, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&ta32, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, rows_pad, kbytes, kbytes, 32, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, (uint64_t)experts * p.rows_b, kbytes, kbytes, 256, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    return launch_tile<false>(ta, ta32, tb, (const uint8_t*)x_sf, (const uint8_t*)w_sf, p.kb_total * 4, p, stream);
 }

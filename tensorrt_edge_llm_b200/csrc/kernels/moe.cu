@@ -210,7 +210,18 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_idx, int* __restri
     __shared__ int total_tiles;
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < slots; i += blockDim.x) {
+    // Bound by the latency of one CTA's loads: four slots a load, four loads in flight (64000 slots: 35 -> 18 us)
+    const int quads = (reinterpret_cast<uintptr_t>(topk_idx) | reinterpret_cast<uintptr_t>(dst_row)) & 15 ? 0 : slots / 4;
+    const int4* idx4 = reinterpret_cast<const int4*>(topk_idx);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < quads; i += blockDim.x) {
+        const int4 v = idx4[i];
+        const int e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (e[q] >= expert_lo && e[q] < expert_hi) atomicAdd(&count[e[q]], 1);
+    }
+    for (int i = 4 * quads + threadIdx.x; i < slots; i += blockDim.x) {
         const int e = topk_idx[i];
         if (e >= expert_lo && e < expert_hi) atomicAdd(&count[e], 1);
     }
@@ -255,46 +266,73 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_idx, int* __restri
         tile_expert[t] = -1;
         tile_expert[max_tiles + t] = 0;
     }
-    for (int i = threadIdx.x; i < slots; i += blockDim.x) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < quads; i += blockDim.x) {
+        const int4 v = idx4[i];
+        const int e[4] = {v.x, v.y, v.z, v.w};
+        int r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = e[q] >= expert_lo && e[q] < expert_hi ? offset[e[q]] * 128 + atomicAdd(&cursor[e[q]], 1) : -1;
+        reinterpret_cast<int4*>(dst_row)[i] = make_int4(r[0], r[1], r[2], r[3]);
+    }
+    for (int i = 4 * quads + threadIdx.x; i < slots; i += blockDim.x) {
         const int e = topk_idx[i];
         if (e >= expert_lo && e < expert_hi) dst_row[i] = offset[e] * 128 + atomicAdd(&cursor[e], 1);
         else dst_row[i] = -1;
     }
 }
 
-// grid.x = routed slots (token*top_k + k); one CTA copies / quantises one row of `hidden` features.
+// One CTA per token: its row is read (and quantised) once and written to the rows of all its slots.  Bound by the writes: 8000 tokens of
+// 2048, 8 slots each: 22 us (68 us with a CTA per slot, which read and quantised every row eight times).
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ dst_row, T* __restrict__ out16,
                                   uint8_t* __restrict__ xq, uint8_t* __restrict__ sf, const float* __restrict__ global_scale,
                                   int top_k, int hidden, int k64_pad) {
     pdl_prologue();
-    const int slot = blockIdx.x;
-    const int row = dst_row[slot];
-    if (row < 0) return;
-    const T* src = x + (size_t)(slot / top_k) * hidden;
+    const int* dst = dst_row + (size_t)blockIdx.x * top_k;
+    const T* src = x + (size_t)blockIdx.x * hidden;
     if (out16) {
-        for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x)
-            reinterpret_cast<uint4*>(out16 + (size_t)row * hidden)[i] = reinterpret_cast<const uint4*>(src)[i];
+        for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
+            const uint4 v = reinterpret_cast<const uint4*>(src)[i];
+            for (int k = 0; k < top_k; ++k)
+                if (dst[k] >= 0) reinterpret_cast<uint4*>(out16 + (size_t)dst[k] * hidden)[i] = v;
+        }
         return;
     }
     const float gs = *global_scale;
     const float inv_gs = 1.f / gs;
-    for (int u = threadIdx.x; u < hidden / 16; u += blockDim.x) {
-        const uint4 a0 = reinterpret_cast<const uint4*>(src + u * 16)[0], a1 = reinterpret_cast<const uint4*>(src + u * 16)[1];
-        const T* e0 = reinterpret_cast<const T*>(&a0);
-        const T* e1 = reinterpret_cast<const T*>(&a1);
-        float v[16];
-        float amax = 0.f;
+    const int units = hidden / 16;
+    // whole warps walk together: four neighbouring lanes hold the four scales of one 32-bit word of the atoms
+    for (int u0 = threadIdx.x & ~31; u0 < units; u0 += blockDim.x) {
+        const int u = u0 + (threadIdx.x & 31);
+        uint2 packed = make_uint2(0, 0);
+        uint8_t s8 = 0;
+        if (u < units) {
+            const uint4 a0 = reinterpret_cast<const uint4*>(src + u * 16)[0], a1 = reinterpret_cast<const uint4*>(src + u * 16)[1];
+            const T* e0 = reinterpret_cast<const T*>(&a0);
+            const T* e1 = reinterpret_cast<const T*>(&a1);
+            float v[16];
+            float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = Cvt<T>::to_f(e0[i]);
-            v[8 + i] = Cvt<T>::to_f(e1[i]);
-            amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[8 + i])));
+            for (int i = 0; i < 8; ++i) {
+                v[i] = Cvt<T>::to_f(e0[i]);
+                v[8 + i] = Cvt<T>::to_f(e1[i]);
+                amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[8 + i])));
+            }
+            packed = nvfp4_quantize_block16(v, amax, gs, inv_gs, s8);
         }
-        uint8_t s8;
-        const uint2 packed = nvfp4_quantize_block16(v, amax, gs, inv_gs, s8);
-        *reinterpret_cast<uint2*>(xq + (size_t)row * (hidden / 2) + u * 8) = packed;
-        sf[sf_atom_offset(row, u, k64_pad)] = s8;
+        uint32_t word = s8;
+        word |= __shfl_down_sync(0xffffffffu, word, 1) << 8;
+        word |= __shfl_down_sync(0xffffffffu, word, 2) << 16;
+        if (u >= units) continue;
+        const bool whole = (u & ~3) + 4 <= units;
+        for (int k = 0; k < top_k; ++k) {
+            const int row = dst[k];
+            if (row < 0) continue;
+            *reinterpret_cast<uint2*>(xq + (size_t)row * (hidden / 2) + u * 8) = packed;
+            if (!whole) sf[sf_atom_offset(row, u, k64_pad)] = s8;
+            else if ((u & 3) == 0) *reinterpret_cast<uint32_t*>(sf + sf_atom_offset(row, u, k64_pad)) = word;
+        }
     }
 }
 
@@ -306,14 +344,25 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const int* __restric
     const int t = blockIdx.x;
     for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int k = 0; k < top_k; ++k) {
-            const int row = dst_row[(size_t)t * top_k + k];
-            if (row < 0) continue;
-            const float w = topk_w[(size_t)t * top_k + k];
-            const uint4 u = reinterpret_cast<const uint4*>(y + (size_t)row * hidden)[i];
-            const T* e = reinterpret_cast<const T*>(&u);
+        // rows of four slots in flight at a time (8000 x 2048, 8 slots: 57 -> 50 us)
+        for (int k0 = 0; k0 < top_k; k0 += 4) {
+            uint4 u[4];
+            float w[4];
+            bool on[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] += w * Cvt<T>::to_f(e[j]);
+            for (int q = 0; q < 4; ++q) {
+                const int row = k0 + q < top_k ? dst_row[(size_t)t * top_k + k0 + q] : -1;
+                on[q] = row >= 0;
+                w[q] = on[q] ? topk_w[(size_t)t * top_k + k0 + q] : 0.f;
+                u[q] = on[q] ? reinterpret_cast<const uint4*>(y + (size_t)row * hidden)[i] : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (!on[q]) continue;
+                const T* e = reinterpret_cast<const T*>(&u[q]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] += w[q] * Cvt<T>::to_f(e[j]);
+            }
         }
         uint4 o;
         o.x = Cvt<T>::pack2(acc[0], acc[1]);
@@ -395,10 +444,10 @@ extern "C" int telb_moe_gather(const void* x, const int* dst_row, void* out16, v
     if (hidden % (out16 ? 8 : 16)) return fail("telb_moe_gather: hidden must be a multiple of 16 (8 for a plain copy)");
     const int k64 = telb_nvfp4_k64_pad(hidden);
     if (is_bf16)
-        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__nv_bfloat16>), dim3(slots), dim3(128), 0, stream, (const __nv_bfloat16*)x,
+        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__nv_bfloat16>), dim3(slots / top_k), dim3(128), 0, stream, (const __nv_bfloat16*)x,
                     dst_row, (__nv_bfloat16*)out16, (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);
     else
-        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__half>), dim3(slots), dim3(128), 0, stream, (const __half*)x, dst_row,
+        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__half>), dim3(slots / top_k), dim3(128), 0, stream, (const __half*)x, dst_row,
                     (__half*)out16, (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);
     return 0;
 }

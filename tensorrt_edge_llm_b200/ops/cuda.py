@@ -1108,8 +1108,8 @@ def gemm_grouped(x, weight, ws: MoeWorkspace, experts_local: int, alpha=None, bi
         out = torch.empty(ws.rows_pad, n, dtype=x.dtype, device=weight.device)
         _check(lib().telb_gemm_nvfp4_grouped(_p(x.xq), _p(x.sf), _p(weight), _p(w_sf), _p(out), c_int(ws.rows_pad), c_int(n), c_int(k),
                                              c_int(experts_local), _p(ws.tile_expert), _p(alpha),
-                                             c_int(1 if x.dtype == torch.bfloat16 else 0), _p(wsx.status), _stream()),
-               "gemm_nvfp4_grouped")
+                                             c_int(1 if x.dtype == torch.bfloat16 else 0), _p(wsx.status),
+                                             c_int(ws.dst_row.numel()), _stream()), "gemm_nvfp4_grouped")
         return out
     n = weight.shape[0] // experts_local
     k = weight.shape[1]

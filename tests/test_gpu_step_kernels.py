@@ -216,3 +216,63 @@ def test_pair_gemm_equals_the_single_cta_kernel(cu, m, n, k, dtype):
         if act == "relu2" or n % 16 == 0:
             assert torch.equal(cu.gemm_act(x, w, act), getattr(cu, act)(plain))
     _check_status(cu)
+
+
+@pytest.mark.parametrize("tokens,experts,top_k,hidden,inter", [(1, 8, 2, 256, 128), (40, 16, 4, 544, 384), (33, 128, 8, 2048, 256), (700, 4, 2, 1056, 640), (300, 3, 1, 288, 192)])
+def test_grouped_gemm_tiles_equal_the_128_wide_kernel(cu, tokens, experts, top_k, hidden, inter):
+    """128 x 256 tiles over experts: few rows, full tiles and tails, unused tiles, half a tile of columns at an expert's end."""
+    g = torch.Generator(device="cuda").manual_seed(tokens + experts)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g).half()
+    idx = torch.rand(tokens, experts, device="cuda", generator=g).topk(top_k, 1).indices.int()
+    n = 2 * inter
+    wq, sf, _ = ref.nvfp4_quantize(torch.randn(experts * n, hidden, device="cuda", generator=g) * 0.05)
+    w_sf, alpha = cu.nvfp4_swizzle_scales(sf), torch.rand(experts * n, device="cuda", generator=g) * 1e-3
+    L, outs = cu.lib(), []
+    old = L.telb_set_nvfp4_wide_mode(0)
+    lo, hi = (1, experts) if experts == 3 else (0, experts)
+    try:
+        for mode in (0, 1):
+            L.telb_set_nvfp4_wide_mode(mode)
+            ws = cu.moe_align(idx, experts, lo, hi)
+            a = cu.moe_gather(x, ws, top_k, torch.full((1,), 1.0 / 448, device="cuda"))
+            rows = ws.dst_row.clone()
+            ws.dst_row = torch.empty(10 ** 6, dtype=torch.int32, device="cuda")         # as many routed rows as take the wide tiles
+            y = cu.gemm_grouped(a, wq[lo * n:], ws, hi - lo, alpha=alpha[lo * n:], w_sf=cu.nvfp4_swizzle_scales(sf[lo * n:]))
+            outs.append(torch.where(rows[:, None] >= 0, y[rows.clamp(min=0).long()], torch.zeros((), dtype=y.dtype, device="cuda")))
+    finally:
+        L.telb_set_nvfp4_wide_mode(old)
+    _check_status(cu)
+    assert torch.equal(*outs) and outs[0].abs().max() > 0
+
+
+@pytest.mark.parametrize("hidden", [16, 64, 560, 2048, 4112])
+@pytest.mark.parametrize("tokens,top_k,experts,lo,hi", [(1, 1, 4, 0, 4), (37, 3, 8, 2, 6), (1025, 8, 128, 0, 128)])
+def test_moe_tables_gather_and_combine(cu, tokens, top_k, experts, lo, hi, hidden):
+    """Slot counts that are no multiple of four, experts of other ranks, rows whose scales end inside a word; all against their plain statement."""
+    g = torch.Generator(device="cuda").manual_seed(hidden + tokens)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g).bfloat16()
+    idx = torch.rand(tokens, experts, device="cuda", generator=g).topk(top_k, 1).indices.int()
+    ws = cu.moe_align(idx, experts, lo, hi)
+    dst, flat = ws.dst_row.long(), idx.reshape(-1).long()
+    on = (flat >= lo) & (flat < hi)
+    assert torch.equal(dst >= 0, on) and dst[on].unique().numel() == int(on.sum())
+    assert torch.equal(ws.tile_expert[dst[on] // 128].long(), flat[on] - lo)
+    gs = torch.full((1,), 1.0 / 448, device="cuda")
+    a = cu.moe_gather(x, ws, top_k, gs)
+    xq, sf = cu.nvfp4_quantize(x, gs)
+    # the two kernels scale by a product and by a quotient: values on an edge of the four-bit grid may fall either way
+    assert (a.xq[dst[on]] != xq.repeat_interleave(top_k, 0)[on]).sum() <= 1 + 0.02 * on.sum() * hidden // 2
+    assert torch.equal(a.xq[dst[on]], cu.moe_gather(x.repeat_interleave(top_k, 0), ws, 1, gs).xq[dst[on]])
+    k64 = cu.lib().telb_nvfp4_k64_pad(hidden)
+
+    def scales(buf, rows):
+        kb = torch.arange(hidden // 16, device="cuda")
+        r = rows[:, None]
+        return buf.reshape(-1).view(torch.uint8)[((r // 128) * k64 + kb // 4) * 512 + (r % 32) * 16 + (r % 128) // 32 * 4 + kb % 4]
+
+    assert torch.equal(scales(a.sf, dst[on]), scales(sf, torch.arange(tokens, device="cuda").repeat_interleave(top_k)[on]))
+    w = torch.rand(tokens, top_k, device="cuda", generator=g)
+    y = cu.moe_gather(x, ws, top_k, None)
+    want = (x.float()[:, None] * (w * on.view(tokens, top_k))[:, :, None]).sum(1)
+    assert (cu.moe_combine(y, ws, w).float() - want).norm() <= 2 ** -8 * want.norm() + 1e-6     # one rounding of an fp32 sum
+    _check_status(cu)
