@@ -242,8 +242,9 @@ using namespace telb;
 // Whether M x N outputs take the pair kernel.  Both kernels work in whole waves of tiles (74 pairs of 256 x 256, 148 CTAs of 128 x 256);
 // a pair's wave takes 0.82 of the single CTA's (8129 x 24576 x 4096: 42 waves, 1035 against 1270 us), so it pays unless the larger tile
 // needs that many more waves: 1030 x 24576 x 4096: 7 against 6 waves, 203 against 216 us; 1030 x 4096 x 12288: 2 against 1, 173 against 102 us.
-extern "C" int telb_gemm_pair_pays(int M, int N) {
-    if (M <= 128 || N < 256) return 0;
+extern "C" int telb_gemm_skinny_pays(int M, int N, int K);
+extern "C" int telb_gemm_pair_pays(int M, int N, int K) {
+    if (M <= 128 || N < 256 || telb_gemm_skinny_pays(M, N, K)) return 0;
     const long long sms = sm_count(), nb = (N + 255) / 256;
     const long long pair = ((M + 255) / 256 * nb + sms / 2 - 1) / (sms / 2), single = ((M + 127) / 128 * nb + sms - 1) / sms;
     return pair * 82 < single * 100;

@@ -1,4 +1,4 @@
-// Decode-size GEMM (M <= 128 tokens):  out[M,N] = x[M,K] · w[N,K]ᵀ · alpha (+bias, +residual),
+// Decode-size GEMM (M <= 128 tokens, 16-bit operands up to 256):  out[M,N] = x[M,K] · w[N,K]ᵀ · alpha (+bias, +residual),
 // for 16-bit weights and for NVFP4 block-scaled weights/activations.
 //
 // A decode step is bound by streaming the weights once, and each projection is only a few
@@ -13,6 +13,10 @@
 //     its weight-tile TMA loads immediately (weights never depend on the predecessor) and executes
 //     `griddepcontrol.wait` only before touching activations or writing outputs.
 // No TMA load here uses cluster multicast: every CTA fetches its own K-slice.
+//
+// 129 to 256 tokens (small prompts, tree verification): one CTA per SM with 48 KB stages.  A prompt-size tile leaves most SMs without work
+// there; the K split fills them without a workspace (240 x 4096 x 12288: 33 us against 60 in 256 x 256 tiles; 240 x 4096 x 4096: 20 against
+// 24).  This form waits for the kernel before it touches the weights: at these sizes they may be a temporary that it has just expanded.
 //
 // Tensor-parallel fusion at decode size (both optional, same contract as the large-M kernels):
 //   * reduce-scatter epilogue: the output row of token t belongs to rank t / rows_per_rank and is stored straight
@@ -127,7 +131,7 @@ struct SkinnyCfg {
     static constexpr int kSf = KIND == 1 ? 2 * 2048 : (KIND == 2 ? 4096 : 0);      // NVFP4 scale atoms, or the packed INT4 tile
     static constexpr int kStage = kWTile + kXTile + kSf;
     static constexpr int kRed = BN * kBM * 4;                                // fp32 partial tile
-    static constexpr int kBudget = 98304;
+    static constexpr int kBudget = BN > 128 ? 196608 : 98304;      // one CTA per SM, or two
     static constexpr int kStagesRaw = kBudget / kStage;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : (kStagesRaw < 2 ? 2 : kStagesRaw);
     static constexpr int kSmemData = kStages * kStage > kRed ? kStages * kStage : kRed;
@@ -225,6 +229,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             // Weight tiles (and their scales) of the first ring pass do not depend on the previous
             // kernel: issue them before waiting for it.
             const int pre = min(nkb, STAGES);
+            if constexpr (BN > 128) pdl_wait();
             for (int j = 0; j < pre; ++j) {
                 uint8_t* sw = smem + j * Cfg::kStage;
                 if constexpr (KIND == 2) {
@@ -504,6 +509,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             const int items = max(0, c_hi - c_lo) * 32;
             const bool vec_out = (p.n_out & 3) == 0;
             float* fin = red + BN * kBM;            // SwiGLU mode: this CTA's reduced token columns [per][128], local only
+#pragma unroll (BN > 128 ? 4 : 1)
             for (int it = etid; it < items; it += 128) {
                 const int c = c_lo + (it >> 5);
                 const int fg = (it & 31) * 4;
@@ -632,7 +638,14 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const Ski
 // (48 clusters of 6 or 8 do not fit and run as two waves, 48 clusters of 4 do).  Among the sizes that divide the
 // work the estimate below — waves x (K steps per rank + fixed launch-to-first-byte cost) + reduction cost per rank —
 // picks the cheapest; its constants come from timing the Qwen3-8B decode projections with HBM-resident weights.
-static int choose_ranks(int tiles, int kb_total, int force) {
+// `wide` (more than 128 tokens): one CTA per SM, and a K step takes 0.4 us (16 KB of weights per SM at the measured HBM rate).
+static float ranks_estimate(int tiles, int kb_total, int r, bool wide) {
+    const int capacity = 8 * ((wide ? 16 : 32) / r);
+    const int waves = (tiles + capacity - 1) / capacity;
+    const int steps = (kb_total + r - 1) / r;
+    return waves * (steps * (wide ? 0.4f : 0.35f) + 4.0f) + r * 0.15f;
+}
+static int choose_ranks(int tiles, int kb_total, int force, bool wide) {
     if (force > 0) return force > 8 ? 8 : (force > kb_total ? kb_total : force);
     static const int cand[6] = {1, 2, 3, 4, 6, 8};
     int best_r = 1;
@@ -640,10 +653,7 @@ static int choose_ranks(int tiles, int kb_total, int force) {
     for (int i = 0; i < 6; ++i) {
         const int r = cand[i];
         if (r > kb_total) break;
-        const int capacity = 8 * (32 / r);
-        const int waves = (tiles + capacity - 1) / capacity;
-        const int steps = (kb_total + r - 1) / r;
-        const float est = waves * (steps * 0.35f + 4.0f) + r * 0.15f;
+        const float est = ranks_estimate(tiles, kb_total, r, wide);
         if (est < best - 1e-3f) {
             best = est;
             best_r = r;
@@ -661,6 +671,9 @@ static int dispatch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const S
         case 16: TELB_SK(16);
         case 32: TELB_SK(32);
         case 64: TELB_SK(64);
+        case 256:
+            if constexpr (KIND == 0) { TELB_SK(256); }
+            return fail("telb_gemm_skinny: 256 tokens are built for 16-bit operands");
         default: TELB_SK(128);
     }
 #undef TELB_SK
@@ -686,14 +699,14 @@ static int gemm_skinny_impl(int kind, const void* x, const void* x_sf, const voi
                             const SkinnySwiglu* sw = nullptr, int out_f32 = 0) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     if (sw && (M > 64 || N % 128 || residual)) return fail("telb_gemm_skinny: the SwiGLU epilogue needs M <= 64, N % 128 == 0 and no residual");
-    if (M > 128) return fail("telb_gemm_skinny: M must be <= 128");
+    if (M > (kind == 0 && !fusion && !sw ? 256 : 128)) return fail("telb_gemm_skinny: M must be <= 128 (256 for plain 16-bit operands)");
     if (fusion && fusion->rs_world > 1) {
         if (residual) return fail("telb_gemm_skinny: reduce-scatter epilogue takes no residual");
         if (N % 4) return fail("telb_gemm_skinny: reduce-scatter epilogue needs N % 4 == 0");
         if (fusion->rs_world > 8 || fusion->rs_rows_per_rank <= 0 || (long long)fusion->rs_rows_per_rank * fusion->rs_world < M)
             return fail("telb_gemm_skinny: reduce-scatter rows_per_rank * world must cover M (world <= 8)");
     }
-    const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+    const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     SkinnyParams p{};
     p.n_out = N;
     p.m_tok = M;
@@ -752,11 +765,22 @@ static int gemm_skinny_impl(int kind, const void* x, const void* x_sf, const voi
         if (make_tmap_2d(&tx, dt, 2, x, M, K, (uint64_t)K * 2, bn, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
     }
     const int tiles = (N + kBM - 1) / kBM;
-    int ranks = choose_ranks(tiles, p.kb_total, force_ranks);
+    int ranks = choose_ranks(tiles, p.kb_total, force_ranks, bn > 128);
     p.kb_per_rank = (p.kb_total + ranks - 1) / ranks;
     p.ranks = (p.kb_total + p.kb_per_rank - 1) / p.kb_per_rank;
     if (kind == 2) return dispatch_skinny<2>(tw, tx, p, bn, stream);
     return kind == 1 ? dispatch_skinny<1>(tw, tx, p, bn, stream) : dispatch_skinny<0>(tw, tx, p, bn, stream);
+}
+
+// Whether 129 to 256 rows of 16-bit operands are faster split along K here than in prompt-size tiles (74 pairs of 256 x 256, 0.28 us a K
+// step and 6 us around them: 240 x 4096 x 12288 60 us, 240 x 4096 x 4096 24, 240 x 24576 x 4096 54, which stays there).
+extern "C" int telb_gemm_skinny_pays(int M, int N, int K) {
+    if (M <= 128) return 1;
+    if (M > 256) return 0;
+    const int tiles = (N + kBM - 1) / kBM, kb = (K + 63) / 64, pairs = sm_count() / 2;
+    const float own = ranks_estimate(tiles, kb, choose_ranks(tiles, kb, 0, true), true) + 9.f;      // one CTA per SM: nothing of it overlaps
+    const float pair = (((N + 255) / 256 + pairs - 1) / pairs) * kb * 0.28f + 6.f;
+    return own < pair;
 }
 
 extern "C" int telb_gemm_skinny_fused(int kind, const void* x, const void* x_sf, const void* w, const void* w_sf, void* out, int M,

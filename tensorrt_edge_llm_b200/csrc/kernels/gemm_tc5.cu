@@ -186,7 +186,8 @@ extern "C" int telb_gemm_skinny_fused(int kind, const void* x, const void* x_sf,
 extern "C" int telb_gemm_skinny_f32out(const void* x, const void* w, float* out, int M, int N, int K, const float* bias, int is_bf16,
                                        int* status, cudaStream_t stream);
 
-extern "C" int telb_gemm_pair_pays(int M, int N);
+extern "C" int telb_gemm_pair_pays(int M, int N, int K);
+extern "C" int telb_gemm_skinny_pays(int M, int N, int K);
 extern "C" int telb_gemm_pair(const void* x, const void* w, void* out, int M, int N, int K, const void* bias, const float* alpha,
                               const void* residual, int epi, int is_bf16, int* status, cudaStream_t stream);
 
@@ -210,9 +211,9 @@ static int gemm_f16_impl(const void* x, const void* w, void* out, int M, int N, 
     if (fusion) mode = 1;         // otherwise the fused collectives run in the large-M layout
     if (mode == 0 && M <= 128 && out_f32)
         return telb_gemm_skinny_f32out(x, w, (float*)out, M, N, K, (const float*)bias, is_bf16, status, stream);
-    if (mode == 0 && M <= 128)
+    if (mode == 0 && !out_f32 && telb_gemm_skinny_pays(M, N, K))
         return telb_gemm_skinny(0, x, nullptr, w, nullptr, out, M, N, K, alpha, bias, residual, is_bf16, status, 0, stream);
-    if (mode == 0 && !out_f32 && telb_gemm_pair_pays(M, N))
+    if (mode == 0 && !out_f32 && telb_gemm_pair_pays(M, N, K))
         return telb_gemm_pair(x, w, out, M, N, K, bias, alpha, residual, 0, is_bf16, status, stream);
     const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const bool swapped = mode == 2 || (mode == 0 && M <= 128);

@@ -325,7 +325,7 @@ def gemm_act(x: torch.Tensor, weight: torch.Tensor, act: str) -> torch.Tensor:
     m, k = x.shape
     n, rows = weight.shape[0] // (2 if act == "swiglu" else 1), weight.shape[0]
     if not (k % 8 == 0 and n % 8 == 0 and weight.dtype == x.dtype and x.dtype != torch.float32 and x.is_contiguous() and weight.is_contiguous()
-            and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and lib().telb_gemm_pair_pays(c_int(m), c_int(rows))):
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and lib().telb_gemm_pair_pays(c_int(m), c_int(rows), c_int(k))):
         y = gemm(x, weight)
         return swiglu(y) if act == "swiglu" else relu2(y)
     out = torch.empty(m, n, dtype=x.dtype, device=x.device)

@@ -276,3 +276,19 @@ def test_moe_tables_gather_and_combine(cu, tokens, top_k, experts, lo, hi, hidde
     want = (x.float()[:, None] * (w * on.view(tokens, top_k))[:, :, None]).sum(1)
     assert (cu.moe_combine(y, ws, w).float() - want).norm() <= 2 ** -8 * want.norm() + 1e-6     # one rounding of an fp32 sum
     _check_status(cu)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,ranks", [(129, 128, 8, 1), (256, 4096, 4096, 0), (200, 1000, 1032, 3), (240, 520, 12288, 8), (131, 6, 256, 2), (255, 3000, 520, 1)])
+def test_split_gemm_of_129_to_256_rows(cu, m, n, k, ranks, dtype):
+    """One token tile of 256: ragged tokens, features and K steps, every way out of the epilogue; bias, scale and residual."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x, w = torch.randn(m, k, device="cuda", generator=g).to(dtype), (torch.randn(n, k, device="cuda", generator=g) * k ** -0.5).to(dtype)
+    bias, res = torch.randn(n, device="cuda", generator=g).to(dtype), torch.randn(m, n, device="cuda", generator=g).to(dtype)
+    alpha, exact = torch.rand(n, device="cuda", generator=g), x.double() @ w.double().t()
+    for kw, want in ((dict(), exact), (dict(alpha=alpha, bias=bias, residual=res), exact * alpha.double() + bias.double() + res.double())):
+        got = cu.gemm_skinny(x, w, ranks=ranks, **kw)
+        eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+        assert ((got.double() - want).abs() <= eps * want.abs() + 1e-5 * want.abs().max()).all()      # one rounding of an fp32 sum
+        assert ((cu.gemm(x, w, **kw).double() - want).abs() <= eps * want.abs() + 1e-5 * want.abs().max()).all()
+    _check_status(cu)
