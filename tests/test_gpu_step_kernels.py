@@ -292,3 +292,12 @@ def test_split_gemm_of_129_to_256_rows(cu, m, n, k, ranks, dtype):
         assert ((got.double() - want).abs() <= eps * want.abs() + 1e-5 * want.abs().max()).all()      # one rounding of an fp32 sum
         assert ((cu.gemm(x, w, **kw).double() - want).abs() <= eps * want.abs() + 1e-5 * want.abs().max()).all()
     _check_status(cu)
+
+
+@pytest.mark.parametrize("seqs,past", [(1, 9000), (3, 2300), (9, 1100), (20, 2100), (25, 2100), (40, 300)])
+def test_decode_attention_with_chosen_splits(cu, seqs, past):
+    q, kv, meta = _paged_step([1] * seqs, [past - 37 * i for i in range(seqs)] if past > 37 * seqs else [past] * seqs, 32, 8, 64, torch.bfloat16)
+    want = ref.paged_attention(q, kv, meta, 128 ** -0.5)
+    got = cu.paged_attention(q, kv, meta, 128 ** -0.5)
+    assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm()       # probabilities and outputs rounded to 16 bits
+    _check_status(cu)
