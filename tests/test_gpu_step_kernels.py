@@ -301,3 +301,28 @@ def test_decode_attention_with_chosen_splits(cu, seqs, past):
     got = cu.paged_attention(q, kv, meta, 128 ** -0.5)
     assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm()       # probabilities and outputs rounded to 16 bits
     _check_status(cu)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens,hq,hkv,norm", [(256, 4, 1, True), (300, 5, 5, False), (700, 32, 8, True), (5000, 3, 1, True)])
+def test_rope_rows_of_several_heads_a_warp(cu, tokens, hq, hkv, norm, dtype):
+    """Head counts that end inside a group of four, one to all groups a warp, sequences and pages that end anywhere."""
+    from tensorrt_edge_llm_b200.ops import build_step_meta, rope_cos_sin
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    q_lens, pasts = [tokens - 101, 1, 100], [3, 70, 0]
+    n = [-(-(a + b) // 64) for a, b in zip(q_lens, pasts)]
+    table = torch.full((3, max(n)), -1, dtype=torch.int32)
+    for i in range(3):
+        table[i, :n[i]] = torch.arange(sum(n[:i]), sum(n[:i + 1]), dtype=torch.int32)
+    meta = build_step_meta(q_lens, pasts, table, 64, device="cuda")
+    qkv = torch.randn(tokens, (hq + 2 * hkv) * 128, device="cuda", generator=g).to(dtype)
+    w = [(torch.rand(128, device="cuda", generator=g) + 0.5).to(dtype) if norm else None for _ in range(2)]
+    cs = rope_cos_sin(8192, 128, 1e6, device="cuda")
+    kv, kv_ref = (torch.zeros(sum(n), 2, hkv, 64, 128, device="cuda", dtype=dtype) for _ in range(2))
+    q = cu.rope_kv_write(qkv, kv, meta, cs, hq, hkv, 128, *w, 1e-6)
+    q_ref = ref.rope_kv_write(qkv, kv_ref, meta, cs, hq, hkv, 128, *w, 1e-6)
+    _check_status(cu)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, b in ((q, q_ref), (kv, kv_ref)):
+        assert (a.float() - b.float()).norm() < 2 * eps * b.float().norm()          # up to three 16-bit roundings, two of which may flip
+    assert torch.equal(kv == 0, kv_ref == 0)
