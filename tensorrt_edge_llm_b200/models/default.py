@@ -18,6 +18,7 @@ from typing import List, Optional, Tuple
 
 import torch
 from torch import nn
+from torch.nn.modules import module as _module
 
 from .. import ops
 from ..config import ModelConfig
@@ -374,9 +375,11 @@ class MLP(nn.Module):
                     return self.down_proj(gp.forward_swiglu(x, scale))
                 return self.down_proj(ops.swiglu(gp(x), scale, interleaved=True))
         gated, scale = self.act in ("silu", "swiglu"), self.down_proj.fused_input_scale()
-        # plain 16-bit rows and weights (no adapter, collective or bias between product and activation)
+        # plain 16-bit rows and weights (no adapter, collective or bias between product and activation), and nobody who watches the projection:
+        # hooks (calibration collects inputs with them) and a replaced forward need the module to be called
         if (type(gp) is Linear and scale is None and gp.bias is None and gp.rs_comm is None and isinstance(x, torch.Tensor) and x.dim() == 2
-                and getattr(x, "ag_wait", None) is None):
+                and x.is_cuda and getattr(x, "ag_wait", None) is None and "forward" not in gp.__dict__
+                and not (gp._forward_hooks or gp._forward_pre_hooks or _module._global_forward_hooks or _module._global_forward_pre_hooks)):
             return self.down_proj(ops.linear_act(x, gp.weight, "swiglu" if gated else "relu2"))
         gu = gp(x)
         return self.down_proj(ops.swiglu(gu, scale) if gated else ops.relu2(gu))
