@@ -267,7 +267,7 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                 if (mask_row) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        // columns below `past` are visible, the others as the row's bits say
+                        // columns below `past` are visible, the others as the row's bits say; a window cuts both
                         const int n0 = c0 + c * 32 - past;           // new-token index of the chunk's first column
                         uint32_t vis = 0;
                         if (n0 < qlen) {
@@ -283,6 +283,8 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                             }
                             if (qlen - n0 < 32) vis &= (1u << (qlen - n0)) - 1u;
                         }
+                        const int hidden = first_vis - (c0 + c * 32);        // columns of the chunk that lie before the window
+                        if (hidden > 0) vis = hidden < 32 ? vis & (0xffffffffu << hidden) : 0u;
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
                             if (!((vis >> i) & 1u)) s[c][i] = 0xff800000u;

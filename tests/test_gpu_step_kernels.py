@@ -190,6 +190,19 @@ def test_two_tile_attention_of_tree_rows(cu, q_lens, past_lens):
     _check_status(cu)
 
 
+@pytest.mark.parametrize("page", [64, 128])
+@pytest.mark.parametrize("q_lens,past_lens", [([60, 60], [2048, 100]), ([33, 7, 64, 90], [63, 640, 65, 301]), ([1, 200], [700, 0])])
+def test_two_tile_attention_of_tree_rows_in_a_window(cu, q_lens, past_lens, page):
+    """A row sees the keys that its bits and the window both allow: windows shorter than the tree, of several tiles, and longer than the rest."""
+    q, kv, meta = _paged_step(q_lens, past_lens, 32, 8, page, torch.bfloat16, rows_masked=True)
+    for window in (20, 40, 100, 200, 5000):
+        want = ref.paged_attention(q, kv, meta, 128 ** -0.5, sliding_window=window)
+        for kw in (dict(), dict(splits=1), dict(splits=4), dict(kernel="tile")):
+            got = cu.paged_attention(q, kv, meta, 128 ** -0.5, sliding_window=window, **kw)
+            assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm(), (window, kw)
+    _check_status(cu)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k", [(129, 264, 8), (256, 512, 64), (257, 1040, 136), (700, 3000, 200), (5000, 2064, 520)])
 def test_pair_gemm_equals_the_single_cta_kernel(cu, m, n, k, dtype):
