@@ -50,15 +50,17 @@ def _run(cmd: List[str]) -> str:
 # Kernel sources of one model family, for a process that serves only that family from a tree without built libraries: they link
 # into a library of their own (`libtelb_kernels-<family>.so`) in a fraction of the time of the whole set.
 KERNEL_SETS = {
-    "begupel": ["attention_decode_tc5.cu", "attention_simt.cu", "attention_tc5.cu", "attention_tc5_extra.cu", "channel_delta.cu", "elementwise.cu",
-                "gemm_f32.cu", "gemm_skinny_tc5.cu", "gemm_tc5.cu", "latent.cu", "lightning.cu", "lightning_tc5.cu", "nvfp4_host.cu",
-                "stream_post.cu"],
+    "begupel": ["attention_decode_tc5.cu", "attention_simt.cu", "attention_tc5.cu", "attention_tc5_extra.cu", "attention_wide_tc5.cu",
+                "channel_delta.cu", "elementwise.cu", "gemm_f32.cu", "gemm_pair_tc5.cu", "gemm_skinny_tc5.cu", "gemm_tc5.cu", "latent.cu",
+                "lightning.cu", "lightning_tc5.cu", "nvfp4_host.cu", "stream_post.cu"],
     "debonex": ["attention_decode_tc5.cu", "attention_latent_tc5.cu", "attention_simt.cu", "attention_tc5.cu", "attention_tc5_extra.cu",
-                "channel_delta.cu", "elementwise.cu", "gemm_f32.cu", "gemm_skinny_tc5.cu", "gemm_tc5.cu", "latent.cu", "nvfp4_host.cu", "stream_norm.cu"],
-    "ditenex": ["attention_mixed_tc5.cu", "attention_simt.cu", "elementwise.cu", "gemm_f32.cu", "gemm_skinny_tc5.cu", "gemm_tc5.cu", "mixed_heads.cu", "moe.cu",
-                "nvfp4_host.cu", "stream_sandwich.cu"],
-    "dimesun": ["attention_decode_tc5.cu", "attention_simt.cu", "attention_tc5.cu", "attention_tc5_extra.cu", "elementwise.cu", "gemm_f32.cu",
-                "gemm_skinny_tc5.cu", "gemm_tc5.cu", "mlstm.cu", "mlstm_tc5.cu", "moe.cu", "nvfp4_host.cu", "stream_norm.cu"],
+                "attention_wide_tc5.cu", "channel_delta.cu", "elementwise.cu", "gemm_f32.cu", "gemm_pair_tc5.cu", "gemm_skinny_tc5.cu",
+                "gemm_tc5.cu", "latent.cu", "nvfp4_host.cu", "stream_norm.cu"],
+    "ditenex": ["attention_mixed_tc5.cu", "attention_simt.cu", "elementwise.cu", "gemm_f32.cu", "gemm_pair_tc5.cu", "gemm_skinny_tc5.cu",
+                "gemm_tc5.cu", "mixed_heads.cu", "moe.cu", "nvfp4_host.cu", "stream_sandwich.cu"],
+    "dimesun": ["attention_decode_tc5.cu", "attention_simt.cu", "attention_tc5.cu", "attention_tc5_extra.cu", "attention_wide_tc5.cu",
+                "elementwise.cu", "gemm_f32.cu", "gemm_pair_tc5.cu", "gemm_skinny_tc5.cu", "gemm_tc5.cu", "mlstm.cu", "mlstm_tc5.cu",
+                "moe.cu", "nvfp4_host.cu", "stream_norm.cu"],
 }
 
 
