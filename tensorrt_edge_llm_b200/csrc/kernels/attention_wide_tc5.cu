@@ -171,9 +171,13 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
                     for (int h = 0; h < 2; ++h) {
                         int pos = (j0 + j) * 128 + h * 64;
                         if (pos >= kv_end) pos -= 64;            // past the end: rows that the mask hides
-                        const int page = max(table[pos / p.page_size], 0);      // unreserved page: read page 0, the mask hides it
-                        row[h] = (page * 2 * p.hkv + kvh) * p.page_size + pos % p.page_size;
+                        const int page = table[pos / p.page_size];
+                        row[h] = page < 0 ? -1 : (page * 2 * p.hkv + kvh) * p.page_size + pos % p.page_size;
                     }
+                    // A page that a window has retired: its keys are hidden, but its values still enter P V, times zero.  The other half of the
+                    // tile stands in for it, since page 0 holds whatever another sequence wrote.
+                    if (row[0] < 0) row[0] = max(row[1], kvh * p.page_size);
+                    if (row[1] < 0) row[1] = row[0];
                     if (!mbar_wait(&k_empty[stage], ph, abort_flag, p.status, kStatusProducerTimeout)) break;
                     mbar_expect_tx(&k_full[stage], kWideTile);
     #pragma unroll

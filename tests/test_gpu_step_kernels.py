@@ -203,6 +203,21 @@ def test_two_tile_attention_of_tree_rows_in_a_window(cu, q_lens, past_lens, page
     _check_status(cu)
 
 
+@pytest.mark.parametrize("q_lens,past_lens", [([256], [700]), ([40, 300], [1000, 707]), ([90], [164])])
+def test_two_tile_attention_reads_no_page_that_a_window_retired(cu, q_lens, past_lens):
+    """Table entries before the window are -1; page 0, which another sequence may own, holds NaN and must not reach any row."""
+    q, kv, meta = _paged_step(q_lens, past_lens, 32, 8, 64, torch.bfloat16)
+    kv = torch.cat([torch.full_like(kv[:1], float("nan")), kv])
+    meta.page_table = torch.where(meta.page_table >= 0, meta.page_table + 1, meta.page_table)
+    want = ref.paged_attention(q, kv, meta, 128 ** -0.5, sliding_window=100)
+    for i, past in enumerate(past_lens):
+        meta.page_table[i, :(past - 100 + 1) // 64] = -1
+    for splits in (None, 1, 3):
+        got = cu.paged_attention(q, kv, meta, 128 ** -0.5, sliding_window=100, splits=splits)
+        assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm(), splits
+    _check_status(cu)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k", [(129, 264, 8), (256, 512, 64), (257, 1040, 136), (700, 3000, 200), (5000, 2064, 520)])
 def test_pair_gemm_equals_the_single_cta_kernel(cu, m, n, k, dtype):
