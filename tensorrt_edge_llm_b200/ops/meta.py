@@ -15,6 +15,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 
@@ -82,34 +83,36 @@ def build_step_meta(q_lens: Sequence[int], past_lens: Sequence[int], page_table:
     every sequence, for all rows (``logits_all``) or for the listed packed rows (``logits_rows``)."""
     n = len(q_lens)
     q_lens, past_lens = [int(q) for q in q_lens], [int(p) for p in past_lens]
-    i32 = dict(dtype=torch.int32)
-    q, past = torch.tensor(q_lens, **i32), torch.tensor(past_lens, **i32)
-    q_start = torch.zeros(n + 1, **i32)
-    torch.cumsum(q, 0, out=q_start[1:])
+    device = torch.get_default_device() if device is None else torch.device(device)
+    # numpy on the host: a decode step is a few dozen numbers, and a torch call costs several times as much (and would follow a default
+    # device to the GPU)
+    q, past = np.array(q_lens, np.int32), np.array(past_lens, np.int32)
+    q_start = np.zeros(n + 1, np.int32)
+    np.cumsum(q, dtype=np.int32, out=q_start[1:])
     t = int(q_start[n])
-    sid = torch.repeat_interleave(torch.arange(n, **i32), q)
+    sid = np.repeat(np.arange(n, dtype=np.int32), q)
     pos_t = None
     if isinstance(positions, torch.Tensor):          # already on the device (tree steps): no host copy of the values
         pos_t = positions.to(device=device, dtype=torch.int32).reshape(-1)
-        pos = torch.zeros(0, **i32)
+        pos = np.zeros(0, np.int32)
     elif positions is not None:
-        pos = torch.tensor([int(x) for x in positions], **i32)
+        pos = np.array([int(x) for x in positions], np.int32)
     else:
-        pos = torch.arange(t, **i32) + torch.repeat_interleave(past - q_start[:n], q)
+        pos = np.arange(t, dtype=np.int32) + np.repeat(past - q_start[:n], q)
     if logits_rows is not None:
-        lidx = torch.tensor([int(r) for r in logits_rows], **i32)
+        lidx = np.array([int(r) for r in logits_rows], np.int32)
     elif logits_all:
-        lidx = torch.arange(t, **i32)
+        lidx = np.arange(t, dtype=np.int32)
     else:
         lidx = q_start[1:] - 1
-    slots = torch.tensor([int(x) for x in slot_ids] if slot_ids is not None else list(range(n)), **i32)
+    slots = np.array([int(x) for x in slot_ids], np.int32) if slot_ids is not None else np.arange(n, dtype=np.int32)
+    table = page_table.to(torch.int32)
     parts = [q_start, q, past, pos, sid, slots, lidx]
-    table = page_table.to(**i32)
-    if table.device.type == "cpu":
-        parts.append(table)
-    parts = _upload(parts, device)
-    q_start, q, past, pos, sid, slots, lidx = parts[:7]
-    table = parts[7] if len(parts) > 7 else table.to(device)
+    if device.type == "cuda" and table.device.type == "cpu":
+        parts.append(table.detach().reshape(-1).numpy())
+    up = _upload(parts, device)
+    q_start, q, past, pos, sid, slots, lidx = up[:7]
+    table = up[7].view(table.shape) if len(up) > 7 else table.to(device)
     return StepMeta(
         q_start=q_start, q_len=q, past_len=past, positions=pos_t if pos_t is not None else pos, seq_ids=sid, page_table=table, slot_ids=slots,
         logits_idx=lidx, page_size=page_size, num_seqs=n, num_tokens=t, max_q_len=max(q_lens) if n else 0,
@@ -117,14 +120,17 @@ def build_step_meta(q_lens: Sequence[int], past_lens: Sequence[int], page_table:
         tree_mask=tree_mask.to(device) if tree_mask is not None else None, host_lens=tuple(zip(q_lens, past_lens)))
 
 
-def _upload(parts: List[torch.Tensor], device) -> List[torch.Tensor]:
-    """int32 host tensors on ``device``.  To a GPU they travel as one copy from pinned memory that the host does not wait for: a blocking
-    copy per tensor made it wait for the step before and left the GPU idle while this one was put together (0.5 ms of a 3.4 ms step)."""
-    if torch.device(device).type != "cuda":
-        return [p.to(device) for p in parts]
-    sizes = [(p.numel() + 31) // 32 * 32 for p in parts]           # every part starts on 128 bytes
-    host = torch.zeros(sum(sizes), dtype=torch.int32, pin_memory=True)
-    for p, h in zip(parts, host.split(sizes)):
-        h[:p.numel()].copy_(p.reshape(-1))
+def _upload(parts: List[np.ndarray], device: torch.device) -> List[torch.Tensor]:
+    """Flat int32 arrays on ``device``.  To a GPU they travel as one copy from pinned memory that the host does not wait for: a blocking
+    copy per array made it wait for the step before and left the GPU idle while this one was put together (0.5 ms of a 3.4 ms step)."""
+    if device.type != "cuda":
+        return [torch.from_numpy(p).to(device) for p in parts]
+    starts = [0]
+    for p in parts:
+        starts.append(starts[-1] + (p.size + 31) // 32 * 32)       # every part starts on 128 bytes
+    host = torch.empty(starts[-1], dtype=torch.int32, device="cpu", pin_memory=True)
+    flat = host.numpy()
+    for p, at in zip(parts, starts):
+        flat[at:at + p.size] = p
     dev = host.to(device, non_blocking=True)
-    return [d[:p.numel()].view(p.shape) for p, d in zip(parts, dev.split(sizes))]
+    return [dev.narrow(0, at, p.size) for p, at in zip(parts, starts)]
