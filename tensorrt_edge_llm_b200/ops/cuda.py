@@ -164,10 +164,17 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
     return y
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` packed and starting on 16 bytes: a row that is cut out of a wider one counts as contiguous wherever it starts."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 def _rows(t: torch.Tensor):
     """``(tensor, elements from a row to the next)`` of rows ``[T, ...]`` that a kernel reads by 16-byte pieces where they lie: a view into
     wider rows stays one where each row is packed and starts on 16 bytes; everything else is copied."""
     if t.is_contiguous():
+        t = _aligned(t)
         return t, t.stride(0) if t.dim() > 1 and t.shape[0] > 1 else t[0].numel() if t.shape[0] else 0
     packed = t.shape[0] > 0 and t[0].is_contiguous() and t.stride(0) >= t[0].numel()
     if not packed or (t.stride(0) * t.element_size()) % 16 or t.data_ptr() % 16:
@@ -188,11 +195,11 @@ def gated_group_rmsnorm(x, z, weight, n_groups, eps):
 def rmsnorm_gate(x, z, weight, eps):
     """RMS norm of every head of ``x [T, heads, dim]``, times ``silu(z [T, heads * dim])``: ``[T, heads * dim]``."""
     t, heads, dim = x.shape
-    if dim not in (64, 128, 256):
-        n = rmsnorm(x.reshape(t * heads, dim).contiguous(), weight, eps).reshape(t, heads * dim)
+    x, weight = _aligned(x), _aligned(weight)
+    if dim not in (64, 128, 256) or z.dtype != x.dtype:
+        n = rmsnorm(x.reshape(t * heads, dim), weight, eps).reshape(t, heads * dim)
         zf = z.float()
         return (n.float() * (zf * torch.sigmoid(zf))).to(x.dtype)
-    x = x.contiguous()
     z, ldz = _rows(z)
     y = torch.empty(t, heads * dim, dtype=x.dtype, device=x.device)
     _check(lib().telb_rmsnorm_gate(_p(x), _p(z), _p(weight), _p(y), c_ll(t), c_int(heads), c_int(dim), c_ll(ldz), c_float(eps),

@@ -114,6 +114,20 @@ def test_gated_norms_of_rows_in_wider_rows(cu, rows, hidden, groups):
     _check_status(cu)
 
 
+@pytest.mark.parametrize("offset", [1, 3, 8])
+@pytest.mark.parametrize("rows,dim", [(1, 64), (1, 128), (5, 128), (1, 256)])
+def test_gated_head_norm_of_rows_that_start_anywhere(cu, rows, dim, offset):
+    """A row cut out of a wider one is contiguous for torch wherever it starts; gates of another type take the generic form."""
+    g = torch.Generator(device="cuda").manual_seed(dim + offset)
+    r = torch.randn(3, rows * 2 * dim + 16, device="cuda", generator=g).bfloat16()
+    x, w = r[0, offset:offset + rows * 2 * dim].view(rows, 2, dim), r[1, offset:offset + dim]
+    z = torch.randn(rows, 2 * dim + 24, device="cuda", generator=g).bfloat16()[:, offset:offset + 2 * dim]
+    for gate in (z, z.float()):
+        y, yr = cu.rmsnorm_gate(x, gate, w, 1e-5), ref.rmsnorm_gate(x, gate, w, 1e-5)
+        assert (y.float() - yr.float()).norm() < 2 ** -7 * yr.float().norm()        # two 16-bit roundings
+    _check_status(cu)
+
+
 @pytest.mark.parametrize("q_lens,pasts", [([1, 1, 1], [5, 0, 9]), ([3, 1], [0, 4]), ([37, 130], [0, 64]), ([300], [2])])
 def test_recurrences_read_parts_of_wider_rows(cu, q_lens, pasts):
     """x, B, C (q, k, v) and the step sizes as views into one projection's rows give the bits of packed copies."""
