@@ -628,12 +628,35 @@ def _attn_splits(meta: StepMeta, hkv: int, group: int, chunk: int = 0, window: i
     return max(1, min((2 * 148 + ctas - 1) // ctas, kv_tiles, 32))
 
 
+def _two_tile_pays(meta: StepMeta, hkv: int, group: int, window: int = 0) -> bool:
+    """Whether a plain step of head size 128 takes the two-tile kernel, one CTA an SM, or the one-tile kernel, two CTAs an SM.  The lines
+    come from 1516 steps of 1 to 64 sequences, 17 to 2048 rows and up to 8000 cached tokens, of 32 / 8, 16 / 16, 8 / 1 and 32 / 4 heads."""
+    tq = 128 // group
+    ctas = meta.num_seqs * hkv * -(-meta.max_q_len // tq)
+    keys = _visible_len(meta, 0, window)
+    if ctas >= 148 or meta.max_q_len > 4 * tq:
+        # One tile, unsplit.  With few keys a CTA is mostly set-up, which a second one on the SM hides (64 sequences of 60 rows, 32 / 4
+        # heads: 27 us against 42; 32 rows behind 300 cached tokens, 32 / 8: 39 against 49), and so it is while the second tile would
+        # be empty (100 rows behind 600, 16 / 16: 60 against 68).  Steps of which most tiles would be empty stay with the two-tile kernel,
+        # whose grid holds none (47 decode rows beside a prompt of 983: 168 against 70).
+        return 2 * meta.num_tokens < meta.num_seqs * meta.max_q_len or not (keys <= 256 or (meta.max_q_len <= tq and keys <= 768))
+    # One tile, split over the keys.  A handful of tiles splits into shorter pieces than two tiles at a time (60 rows behind 2048, 8 / 1
+    # heads: 12 us against 21), behind long contexts only for few rows, whose many parts are cheap to merge (64 rows behind 8000, 8 / 1: 15
+    # against 23; 32 rows behind 8000, 32 / 8: 24 against 18).  One piece needs no merge (32 rows, 32 / 4: 6.6 against 9.6).
+    few = meta.num_tokens * hkv * group <= 512
+    return not (keys <= 64 or ctas <= 24 and keys > 128 and (keys <= 3072 or few))
+
+
 def _wide_splits(meta: StepMeta, hkv: int, group: int, window: int = 0) -> int:
     """Splits of the two-tile kernel (head size 128): as many as fill the device, one CTA an SM, in one go, of at least 512 keys (a merge
-    of 300 rows cost more than the two thirds of 300 keys that it saved)."""
+    of 300 rows cost more than the two thirds of 300 keys that it saved), where the merge costs less than they save: a tile of 128
+    keys takes 2 us, a merge 2 us and 0.36 ns a split and head row (1024 rows of 16 heads: 24 us in one split, 38 in two)."""
     block = 2 * (128 // group)
     blocks = min(meta.num_tokens // block + meta.num_seqs, meta.num_seqs * -(-meta.max_q_len // block))
-    return max(1, min(148 // max(1, blocks * hkv), _visible_len(meta, 0, window) // 512, 32))
+    keys = _visible_len(meta, 0, window)
+    splits = max(1, min(148 // max(1, blocks * hkv), keys // 512, 32))
+    saved = 2.0 * -(-keys // 128) * (1 - 1 / splits)
+    return splits if 2.0 + 3.6e-4 * splits * meta.num_tokens * hkv * group < saved else 1
 
 
 def _decode_splits(meta: StepMeta, hkv: int, chunk: int = 0, window: int = 0) -> int:
@@ -652,7 +675,8 @@ def paged_attention(q, kv_layer, meta: StepMeta, scale, sliding_window=None, sin
                     skip_thr: Optional[torch.Tensor] = None, skip_stats: Optional[torch.Tensor] = None, chunk: int = 0,
                     fp32_weights: bool = False, back: Optional[tuple] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Paged GQA attention.  Decode-shaped steps (``max_q_len * Hq/Hkv <= 16``, head_dim 128, causal)
-    run the token-major XQA-style kernel; everything else the row-major tile kernel, or its two-tile form for plain steps of head size 128.
+    run the token-major XQA-style kernel; everything else the row-major tile kernel, or its two-tile form for plain steps of head size 128
+    that it suits (all of them where ``splits`` is given).
     ``kernel`` forces ``"decode"`` or ``"tile"`` (one tile a CTA); ``causal=False`` lets every row see every token of its sequence; ``chunk`` > 0 limits
     a row to the keys of its own ``chunk``-token block; ``fp32_weights`` feeds the probabilities to the 16-bit P·V product as high + low
     halves.  fp32 rows and head sizes without a tensor-core form run on the CUDA cores."""
@@ -708,7 +732,8 @@ def paged_attention(q, kv_layer, meta: StepMeta, scale, sliding_window=None, sin
         return out
     if splits is None:
         plain = wide and d == 128 and scale > 0 and sinks is None and skip_thr is None and chunk <= 0 and not fp32_weights and table is None and 128 % group == 0
-        splits = _wide_splits(meta, hkv, group, win) if plain else _attn_splits(meta, hkv, group, chunk, win)
+        wide = plain and _two_tile_pays(meta, hkv, group, win)
+        splits = _wide_splits(meta, hkv, group, win) if wide else _attn_splits(meta, hkv, group, chunk, win)
     _check(lib().telb_paged_attention(
         _p(q), _p(kv_layer), _p(out), _p(meta.q_start), _p(meta.q_len), _p(meta.past_len), _p(meta.page_table),
         _p(tm), c_int(tm.shape[1] if tm is not None else 0), c_int(meta.num_seqs), c_int(t), c_int(meta.max_q_len),

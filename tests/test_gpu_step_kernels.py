@@ -232,6 +232,20 @@ def test_two_tile_attention_reads_no_page_that_a_window_retired(cu, q_lens, past
     _check_status(cu)
 
 
+@pytest.mark.parametrize("q_lens,past_lens,hq,hkv,one_tile", [
+    ([256], [0], 32, 8, True), ([257], [0], 32, 8, False), ([33] * 20, [223] * 20, 32, 8, True), ([33] * 20, [224] * 20, 32, 8, False),
+    ([32] * 20, [736] * 20, 32, 8, True), ([32] * 20, [737] * 20, 32, 8, False), ([60], [2000], 8, 1, True), ([96], [3000], 32, 8, False), ([64], [4000], 8, 1, True), ([31], [0], 32, 8, True),
+    ([96], [900], 32, 8, True), ([97], [900], 32, 8, False), ([100], [0], 16, 16, False), ([1] * 20 + [200], [50] * 21, 32, 8, False),
+    ([1024], [0], 16, 16, False)])
+def test_prompt_attention_on_both_sides_of_the_route(cu, q_lens, past_lens, hq, hkv, one_tile):
+    q, kv, meta = _paged_step(q_lens, past_lens, hq, hkv, 64, torch.bfloat16)
+    want = ref.paged_attention(q, kv, meta, 128 ** -0.5)
+    got, tile = cu.paged_attention(q, kv, meta, 128 ** -0.5), cu.paged_attention(q, kv, meta, 128 ** -0.5, kernel="tile")
+    assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm()
+    assert torch.equal(got, tile) == one_tile
+    _check_status(cu)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k", [(129, 264, 8), (256, 512, 64), (257, 1040, 136), (700, 3000, 200), (5000, 2064, 520)])
 def test_pair_gemm_equals_the_single_cta_kernel(cu, m, n, k, dtype):
