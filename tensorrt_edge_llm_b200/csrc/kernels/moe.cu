@@ -282,8 +282,52 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_idx, int* __restri
     }
 }
 
-// One CTA per token: its row is read (and quantised) once and written to the rows of all its slots.  Bound by the writes: 8000 tokens of
-// 2048, 8 slots each: 22 us (68 us with a CTA per slot, which read and quantised every row eight times).
+// Features 16 u .. 16 u + 15 of a row as NVFP4 codes and their scale.
+template <typename T>
+__device__ __forceinline__ uint2 moe_quantize_unit(const T* __restrict__ src, int u, float gs, float inv_gs, uint8_t& s8) {
+    const uint4 a0 = reinterpret_cast<const uint4*>(src + u * 16)[0], a1 = reinterpret_cast<const uint4*>(src + u * 16)[1];
+    const T* e0 = reinterpret_cast<const T*>(&a0);
+    const T* e1 = reinterpret_cast<const T*>(&a1);
+    float v[16];
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v[i] = Cvt<T>::to_f(e0[i]);
+        v[8 + i] = Cvt<T>::to_f(e1[i]);
+        amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[8 + i])));
+    }
+    return nvfp4_quantize_block16(v, amax, gs, inv_gs, s8);
+}
+
+// One CTA per routed slot (token * top_k + k) copies / quantises one row; nothing is read for a slot of another rank.  For few slots, where
+// launch and latency are all there is, and for one slot a token (see telb_moe_gather).
+template <typename T>
+__global__ void moe_gather_slot_kernel(const T* __restrict__ x, const int* __restrict__ dst_row, T* __restrict__ out16,
+                                       uint8_t* __restrict__ xq, uint8_t* __restrict__ sf, const float* __restrict__ global_scale,
+                                       int top_k, int hidden, int k64_pad) {
+    pdl_prologue();
+    const int slot = blockIdx.x;
+    const int row = dst_row[slot];
+    if (row < 0) return;
+    const T* src = x + (size_t)(slot / top_k) * hidden;
+    if (out16) {
+        for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x)
+            reinterpret_cast<uint4*>(out16 + (size_t)row * hidden)[i] = reinterpret_cast<const uint4*>(src)[i];
+        return;
+    }
+    const float gs = *global_scale;
+    const float inv_gs = 1.f / gs;
+    for (int u = threadIdx.x; u < hidden / 16; u += blockDim.x) {
+        uint8_t s8;
+        const uint2 packed = moe_quantize_unit(src, u, gs, inv_gs, s8);
+        *reinterpret_cast<uint2*>(xq + (size_t)row * (hidden / 2) + u * 8) = packed;
+        sf[sf_atom_offset(row, u, k64_pad)] = s8;
+    }
+}
+
+// One CTA per token: its row is read (and quantised) once and written to the rows of all its slots; a token without a slot of this rank
+// reads nothing.  Bound by the writes: 8000 tokens of 2048, 8 slots each: 22 us (68 us with a CTA per slot, which reads and quantises
+// every row eight times).
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ dst_row, T* __restrict__ out16,
                                   uint8_t* __restrict__ xq, uint8_t* __restrict__ sf, const float* __restrict__ global_scale,
@@ -291,6 +335,10 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
     pdl_prologue();
     const int* dst = dst_row + (size_t)blockIdx.x * top_k;
     const T* src = x + (size_t)blockIdx.x * hidden;
+    int last = -1;
+#pragma unroll 4
+    for (int k = 0; k < top_k; ++k) last = max(last, dst[k]);
+    if (last < 0) return;
     if (out16) {
         for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
             const uint4 v = reinterpret_cast<const uint4*>(src)[i];
@@ -307,20 +355,7 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
         const int u = u0 + (threadIdx.x & 31);
         uint2 packed = make_uint2(0, 0);
         uint8_t s8 = 0;
-        if (u < units) {
-            const uint4 a0 = reinterpret_cast<const uint4*>(src + u * 16)[0], a1 = reinterpret_cast<const uint4*>(src + u * 16)[1];
-            const T* e0 = reinterpret_cast<const T*>(&a0);
-            const T* e1 = reinterpret_cast<const T*>(&a1);
-            float v[16];
-            float amax = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[i] = Cvt<T>::to_f(e0[i]);
-                v[8 + i] = Cvt<T>::to_f(e1[i]);
-                amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[8 + i])));
-            }
-            packed = nvfp4_quantize_block16(v, amax, gs, inv_gs, s8);
-        }
+        if (u < units) packed = moe_quantize_unit(src, u, gs, inv_gs, s8);
         uint32_t word = s8;
         word |= __shfl_down_sync(0xffffffffu, word, 1) << 8;
         word |= __shfl_down_sync(0xffffffffu, word, 2) << 16;
@@ -443,12 +478,23 @@ extern "C" int telb_moe_gather(const void* x, const int* dst_row, void* out16, v
     if (slots <= 0) return 0;
     if (hidden % (out16 ? 8 : 16)) return fail("telb_moe_gather: hidden must be a multiple of 16 (8 for a plain copy)");
     const int k64 = telb_nvfp4_k64_pad(hidden);
-    if (is_bf16)
-        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__nv_bfloat16>), dim3(slots / top_k), dim3(128), 0, stream, (const __nv_bfloat16*)x,
-                    dst_row, (__nv_bfloat16*)out16, (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);
-    else
-        TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<__half>), dim3(slots / top_k), dim3(128), 0, stream, (const __half*)x, dst_row,
-                    (__half*)out16, (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);
+    // A CTA per slot while the slots fit a wave or so (hidden 2048, 8 slots a token, quantised: 32 tokens 2.3 against 2.9 us, 128: 2.8 against
+    // 3.1, 300: 3.8 against 3.5; copied: 64 tokens 2.4 against 2.5, 128: 3.0 against 2.3), and always where a token has only one (5120,
+    // 8000 tokens: 17.5 against 19.3 us; one slot in eight routed here, as an expert-parallel rank receives them: 9.3 against 15.4) or two
+    // copies of its row are made (4096, 8000 tokens: 31.5 against 33.3)
+    const bool by_slot = top_k <= (out16 ? 2 : 1) || slots <= (out16 ? 512 : 1024);
+    const dim3 grid(by_slot ? slots : slots / top_k);
+#define TELB_GATHER(T_)                                                                                                                 \
+    do {                                                                                                                                \
+        if (by_slot)                                                                                                                    \
+            TELB_LAUNCH("moe_gather_slot_kernel", (moe_gather_slot_kernel<T_>), grid, dim3(128), 0, stream, (const T_*)x, dst_row, (T_*)out16, \
+                        (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);                                                  \
+        else                                                                                                                            \
+            TELB_LAUNCH("moe_gather_kernel", (moe_gather_kernel<T_>), grid, dim3(128), 0, stream, (const T_*)x, dst_row, (T_*)out16,    \
+                        (uint8_t*)xq, (uint8_t*)sf, global_scale, top_k, hidden, k64);                                                  \
+    } while (0)
+    if (is_bf16) TELB_GATHER(__nv_bfloat16); else TELB_GATHER(__half);
+#undef TELB_GATHER
     return 0;
 }
 

@@ -334,6 +334,26 @@ def test_moe_tables_gather_and_combine(cu, tokens, top_k, experts, lo, hi, hidde
     _check_status(cu)
 
 
+@pytest.mark.parametrize("hidden", [48, 2048])
+@pytest.mark.parametrize("tokens,top_k", [(128, 8), (129, 8), (64, 8), (65, 8), (1500, 2), (1500, 1)])
+def test_moe_gather_by_slot_and_by_token(cu, tokens, top_k, hidden):
+    """Both sides of the sizes where a CTA per slot gives way to one per token; one expert in eight is here, so most tokens have no slot.  A
+    row per slot, gathered one slot a token, says what every row holds."""
+    g = torch.Generator(device="cuda").manual_seed(hidden + tokens)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g).bfloat16()
+    ws = cu.moe_align(torch.rand(tokens, 16, device="cuda", generator=g).topk(top_k, 1).indices.int(), 16, 4, 6)
+    dst = ws.dst_row.long()
+    on, gs = dst >= 0, torch.full((1,), 1.0 / 448, device="cuda")
+    one, rows = x.repeat_interleave(top_k, 0), dst[dst >= 0]
+    a, b = cu.moe_gather(x, ws, top_k, gs), cu.moe_gather(one, ws, 1, gs)
+    assert torch.equal(a.xq[rows], b.xq[rows])
+    kb = torch.arange(hidden // 16, device="cuda")
+    at = ((rows[:, None] // 128) * cu.lib().telb_nvfp4_k64_pad(hidden) + kb // 4) * 512 + (rows[:, None] % 32) * 16 + (rows[:, None] % 128) // 32 * 4 + kb % 4
+    assert torch.equal(a.sf.reshape(-1).view(torch.uint8)[at], b.sf.reshape(-1).view(torch.uint8)[at])
+    assert torch.equal(cu.moe_gather(x, ws, top_k, None)[rows], one[on])
+    _check_status(cu)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k,ranks", [(129, 128, 8, 1), (256, 4096, 4096, 0), (200, 1000, 1032, 3), (240, 520, 12288, 8), (131, 6, 256, 2), (255, 3000, 520, 1)])
 def test_split_gemm_of_129_to_256_rows(cu, m, n, k, ranks, dtype):
