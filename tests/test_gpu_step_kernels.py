@@ -355,6 +355,24 @@ def test_moe_gather_by_slot_and_by_token(cu, tokens, top_k, hidden):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens,top_k", [(8191, 1), (8195, 1), (4096, 2), (2730, 3), (2731, 3), (1639, 5)])
+def test_moe_tables_and_sums_by_slot_count(cu, tokens, top_k, dtype):
+    """Slot counts around those where the tables are built four slots at a time, with and without a remainder; every batch of the sum."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    idx = torch.rand(tokens, 24, device="cuda", generator=g).topk(top_k, 1).indices.int()
+    ws = cu.moe_align(idx, 24, 3, 21)
+    dst, flat = ws.dst_row.long(), idx.reshape(-1).long()
+    on = (flat >= 3) & (flat < 21)
+    assert torch.equal(dst >= 0, on) and dst[on].unique().numel() == int(on.sum())
+    assert torch.equal(ws.tile_expert[dst[on] // 128].long(), flat[on] - 3)
+    y, w = torch.randn(ws.rows_pad, 72, device="cuda", generator=g).to(dtype), torch.rand(tokens, top_k, device="cuda", generator=g)
+    want = (torch.where(on[:, None], y[dst.clamp(min=0)].double(), 0.0) * w.double().reshape(-1, 1)).view(tokens, top_k, 72).sum(1)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    assert (cu.moe_combine(y, ws, w).double() - want).norm() <= eps * want.norm()             # one rounding of an fp32 sum
+    _check_status(cu)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,n,k,ranks", [(129, 128, 8, 1), (256, 4096, 4096, 0), (200, 1000, 1032, 3), (240, 520, 12288, 8), (131, 6, 256, 2), (255, 3000, 520, 1)])
 def test_split_gemm_of_129_to_256_rows(cu, m, n, k, ranks, dtype):
     """One token tile of 256: ragged tokens, features and K steps, every way out of the epilogue; bias, scale and residual."""
