@@ -477,7 +477,7 @@ extern "C" int telb_gemm_nvfp4_grouped_swiglu(const void* xq, const void* x_sf, 
     return gemm_nvfp4_grouped_impl(xq, x_sf, wq, w_sf, nullptr, rows_pad, N, K, experts, tile_expert, alpha, out_bf16, status, stream, &sw, 0);
 }
 
-// Whether the grouped product takes 128 x 256 tiles.  `slots`: routed rows (0: unknown), of which at most one per expert opens a row tile
+// Whether the grouped product takes 128 x 256 tiles.  `slots`: rows expected here (0: unknown), of which at most one per expert opens a row tile
 // of its own.  From about a wave of wide tiles on they are the faster ones (128 experts of 1536 x 2048 and 2048 x 768, mean of both products:
 // 4 tokens of 8 experts 21.0 -> 15.3 us, 32: 48 -> 32, 1024: 58 -> 46, 8000: 222 -> 138); below, twice as many narrow tiles fill more SMs.
 static bool grouped_takes_tile(int slots, int rows_pad, int experts, int N) {

@@ -1094,10 +1094,12 @@ def clamped_glu(gate_up: torch.Tensor, limit: float, alpha: float, ws: Optional[
 
 class MoeWorkspace:
     """Routing tables of one MoE call over the padded row space (every expert segment is a multiple
-    of 128 rows, so a 128-row tile belongs to exactly one expert)."""
+    of 128 rows, so a 128-row tile belongs to exactly one expert).  ``share``: part of the slots that is expected to be routed to the
+    experts here."""
 
-    def __init__(self, tokens: int, top_k: int, experts_local: int, device):
+    def __init__(self, tokens: int, top_k: int, experts_local: int, device, share: float = 1.0):
         slots = tokens * top_k
+        self.share = share
         self.max_tiles = (slots + 127) // 128 + experts_local
         self.rows_pad = self.max_tiles * 128
         self.dst_row = torch.empty(slots, dtype=torch.int32, device=device)
@@ -1106,9 +1108,10 @@ class MoeWorkspace:
         self.counts = torch.empty(1, dtype=torch.int32, device=device)
 
 
-def moe_align(topk_idx: torch.Tensor, experts: int, expert_lo: int, expert_hi: int) -> MoeWorkspace:
+def moe_align(topk_idx: torch.Tensor, experts: int, expert_lo: int, expert_hi: int, share: Optional[float] = None) -> MoeWorkspace:
+    """``share``: see :class:`MoeWorkspace`; the part of the experts that is here where nothing else is known."""
     t, k = topk_idx.shape
-    ws = MoeWorkspace(t, k, expert_hi - expert_lo, topk_idx.device)
+    ws = MoeWorkspace(t, k, expert_hi - expert_lo, topk_idx.device, (expert_hi - expert_lo) / experts if share is None else share)
     _check(lib().telb_moe_align(_p(topk_idx), _p(ws.dst_row), _p(ws.tile_expert), _p(ws.counts), c_int(t * k), c_int(experts),
                                 c_int(expert_lo), c_int(expert_hi), c_int(ws.max_tiles), _stream()), "moe_align")
     return ws
@@ -1144,7 +1147,7 @@ def gemm_grouped(x, weight, ws: MoeWorkspace, experts_local: int, alpha=None, bi
         _check(lib().telb_gemm_nvfp4_grouped(_p(x.xq), _p(x.sf), _p(weight), _p(w_sf), _p(out), c_int(ws.rows_pad), c_int(n), c_int(k),
                                              c_int(experts_local), _p(ws.tile_expert), _p(alpha),
                                              c_int(1 if x.dtype == torch.bfloat16 else 0), _p(wsx.status),
-                                             c_int(ws.dst_row.numel()), _stream()), "gemm_nvfp4_grouped")
+                                             c_int(max(1, round(ws.dst_row.numel() * ws.share))), _stream()), "gemm_nvfp4_grouped")
         return out
     n = weight.shape[0] // experts_local
     k = weight.shape[1]

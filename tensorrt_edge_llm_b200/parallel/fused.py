@@ -274,7 +274,8 @@ class FusedComm(TorchComm):
         cu._check(cu.lib().telb_ep_wait(cu._p(st.flags), ctypes.c_int(0), ctypes.c_int(world), ctypes.c_void_p(st.epoch.data_ptr()),
                                         cu._p(ws0.status), cu._stream()), "ep_wait")
         n_recv = world * stride
-        ws = cu.moe_align(st.recv_ids.view(-1)[:n_recv].view(n_recv, 1), block.e_local, 0, block.e_local)
+        # every rank's slots are spread over all ranks: about one in `world` of the receive buffer's holds a row
+        ws = cu.moe_align(st.recv_ids.view(-1)[:n_recv].view(n_recv, 1), block.e_local, 0, block.e_local, share=1.0 / world)
         recv = st.recv_rows.view(-1)[:n_recv * hidden].view(n_recv, hidden)
         if block.nvfp4:
             if block._w13_sf is None:
