@@ -8,7 +8,7 @@
 // Each softmax thread owns one cached token, i.e. 16 scores, so the per-tile softmax is a few
 // dozen instructions instead of a row-long loop; the column max is a warp `redux.sync.max.f32`
 // plus one shared-memory exchange, and the column sums are kept as per-thread partials that are
-// reduced once at the end.  O is rescaled lazily (only when a column max grows by more than 2^8).
+// reduced once at the end.  O is rescaled lazily (only when a column max grows by more than 2^8; 2^0.8 with E4M3 probabilities).
 //
 // CTA = (KV head, sequence, KV split); 128-token tiles = 2 pages of 64 (or 1 of 128), fetched by
 // TMA into a 3-stage ring.  Splits write normalised fp32 partials + log-sum-exp; the merge kernel
@@ -136,6 +136,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
     constexpr int kOCol = kSBufs * 16;                          // O accumulators O0, O1 (16 columns each)
     constexpr int kTmemCols = 128;
     constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+    // log2 units by which the running maximum may lag behind: E4M3 probabilities are stored times 256 and end at 448 = 256 x 2^0.807
+    constexpr float kMaxLag = KV8 ? 0.8f : 8.f;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -442,7 +444,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
                     if (c < ncol) {
                         const float mt = fmaxf(fmaxf(red[c], red[16 + c]), fmaxf(red[32 + c], red[48 + c]));
                         const float m_new = fmaxf(m_used[c], mt);
-                        if (m_new > m_used[c] + 8.0f) {               // uniform across the CTA
+                        if (m_new > m_used[c] + kMaxLag) {            // uniform across the CTA
                             f[c] = (m_used[c] == -INFINITY) ? 0.f : exp2f(m_used[c] - m_new);
                             l_part[c] *= f[c];
                             m_used[c] = m_new;

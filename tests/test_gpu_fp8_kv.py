@@ -96,6 +96,24 @@ def test_decode_attention_reads_fp8_pages_in_place(case, dtype):
     cu.Workspace.get(torch.device("cuda", 0)).check_status()
 
 
+@pytest.mark.parametrize("past,hq,hkv", [(700, 32, 8), (2500, 32, 8), (700, 16, 2), (700, 16, 8), (1300, 16, 1)])
+def test_fp8_decode_keeps_probabilities_above_the_first_tiles_maximum(past, hq, hkv):
+    """Later key tiles may hold larger scores than the first: their probabilities, up to the lag of the running maximum above one, must fit
+    E4M3.  A probability rounds by at most 2^-4, whichever its neighbours, over values of either sign."""
+    from tensorrt_edge_llm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(past + hkv)
+    n, most = 3, past // 64 + 1
+    kv = torch.randn(n * most, 2, hkv, 64, 128, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    q = torch.randn(n, hq, 128, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    meta = build_step_meta([1] * n, [past] * n, torch.arange(n * most, dtype=torch.int32).view(n, most), 64, device="cuda")
+    want = ref.paged_attention(q.float(), kv.float(), meta, 128 ** -0.5)
+    for splits in (1, 2, None):
+        got = cu.paged_attention_decode_fp8(q, kv, meta, 128 ** -0.5, None, torch.ones(2, device="cuda"), torch.bfloat16, splits=splits)
+        assert ((got.float() - want).norm(dim=-1) < (2 ** -4 + 2 ** -8) * want.norm(dim=-1)).all(), splits
+    torch.cuda.synchronize()
+    cu.Workspace.get(torch.device("cuda", 0)).check_status()
+
+
 def test_model_with_fp8_kv_tracks_16_bit_cache_eager_and_graph():
     dev = torch.device("cuda", 0)
     cfg = tiny_llama_config(num_hidden_layers=3, vocab_size=512, dtype="bfloat16", head_dim=128, num_attention_heads=4, num_key_value_heads=2,
