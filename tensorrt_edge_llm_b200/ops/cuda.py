@@ -591,7 +591,7 @@ def paged_attention_decode_fp8(q8: torch.Tensor, kv_layer: torch.Tensor, meta: S
     t, hq, d = q8.shape
     hkv = kv_layer.shape[2]
     if splits is None:
-        splits = _decode_splits(meta, hkv)
+        splits = _decode_splits(meta, hkv, fp8=True)
     ws = Workspace.get(q8.device)
     L = lib()
     out = xq = sf = None
@@ -659,14 +659,18 @@ def _wide_splits(meta: StepMeta, hkv: int, group: int, window: int = 0) -> int:
     return splits if 2.0 + 3.6e-4 * splits * meta.num_tokens * hkv * group < saved else 1
 
 
-def _decode_splits(meta: StepMeta, hkv: int, chunk: int = 0, window: int = 0) -> int:
+def _decode_splits(meta: StepMeta, hkv: int, chunk: int = 0, window: int = 0, fp8: bool = False) -> int:
     """Splits of the decode kernel, which keeps two CTAs an SM: as many as fill those 296 places in one go (8 sequences of 4000 tokens: 4
-    splits 28 us, 3 splits 32 us), and three for 148 to 197 items of many tiles, which would leave a third of the places empty (20
-    sequences of 4000: 60 against 72 us; of 700 tokens: 20.5 against 19.1 us)."""
+    splits 30 us, 3 splits 34 us; E4M3 pages 20.5 and 23).  A captured step is planned for the table's capacity, so some of its splits may find
+    no keys; that costs the merge up to 1.3 us (8 sequences of 2 KV heads: 18 splits against 10: 700 tokens 13.1 and 12.0 us, 1500: 13.7 and
+    14.1, 4000: 16.8 and 19.6; one sequence of 8: 32 against 19: 700 tokens 10.7 either way, 8000: 14.8 and 17.9).  148 to 197 items, which
+    leave a third of the places empty, have no merge to begin with and take three splits only where the step's own lengths are known to
+    be long (20 sequences, 16-bit pages: 4000 tokens 65 against 75 us, 700: 21 against 20, 100: 12 against 8; E4M3 pages: 4000 tokens 41
+    against 47, 1500: 23 against 22)."""
     ctas = meta.num_seqs * hkv
     tiles = max(1, (_visible_len(meta, chunk, window) + 127) // 128)
     if ctas >= 148:
-        return 3 if 3 * ctas <= 592 and tiles >= 16 else 1
+        return 3 if meta.host_lens is not None and 3 * ctas <= 592 and tiles >= (24 if fp8 else 16) else 1
     return max(1, min(296 // ctas, tiles, 32))
 
 

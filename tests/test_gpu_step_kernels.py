@@ -397,6 +397,41 @@ def test_decode_attention_with_chosen_splits(cu, seqs, past):
     _check_status(cu)
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("seqs,past,hq,hkv", [(1, 700, 32, 8), (3, 130, 16, 2), (8, 1, 32, 4), (20, 300, 32, 8), (20, 2500, 32, 8)])
+def test_decode_attention_of_steps_planned_for_longer_sequences(cu, seqs, past, hq, hkv, fp8):
+    """A captured step plans its splits for the table's capacity; splits that find no keys add nothing, whatever the scratch held before."""
+    q, kv, meta = _paged_step([1] * seqs, [past + i % 3 for i in range(seqs)], hq, hkv, 64, torch.bfloat16)
+    want = ref.paged_attention(q.to(torch.float8_e4m3fn).bfloat16() if fp8 else q, kv.to(torch.float8_e4m3fn).bfloat16() if fp8 else kv, meta, 128 ** -0.5)
+    sinks = torch.zeros(hq, device="cuda")
+    meta.host_lens, meta.max_seq_len = None, 8192
+    ws = cu.Workspace.get(q.device)
+    for splits in (None, 3, 19, 32):
+        ws.attn_ws.fill_(float("nan"))
+        if fp8:
+            got = cu.paged_attention_decode_fp8(q.to(torch.float8_e4m3fn), kv.to(torch.float8_e4m3fn), meta, 128 ** -0.5, None, torch.ones(2, device="cuda"),
+                                                torch.bfloat16, splits=splits)
+        else:
+            got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits)
+        # probabilities rounded to 16 bits (E4M3: 2^-4 each), outputs to 16, over values of either sign
+        assert (got.float() - want.float()).norm() < (2 ** -4 if fp8 else 8e-3) * want.float().norm(), splits
+        if not fp8:
+            ws.attn_ws.fill_(float("nan"))
+            got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits, sinks=sinks)
+            more = ref.paged_attention(q, kv, meta, 128 ** -0.5, sinks=sinks)
+            assert (got.float() - more.float()).norm() < 8e-3 * more.float().norm(), splits
+    ws.attn_ws.zero_()
+    _check_status(cu)
+
+
+def test_decode_splits_of_known_and_unknown_lengths(cu):
+    """148 to 197 items are split in three only where the step's own lengths are known, and long."""
+    for past, known, fp8, splits in ((2500, True, False, 3), (2500, False, False, 1), (1900, True, False, 1), (2500, True, True, 1), (3100, True, True, 3)):
+        _, _, meta = _paged_step([1] * 20, [past] * 20, 8, 8, 64, torch.bfloat16)
+        meta.host_lens = meta.host_lens if known else None
+        assert cu._decode_splits(meta, 8, fp8=fp8) == splits
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("tokens,hq,hkv,norm", [(256, 4, 1, True), (300, 5, 5, False), (700, 32, 8, True), (5000, 3, 1, True)])
 def test_rope_rows_of_several_heads_a_warp(cu, tokens, hq, hkv, norm, dtype):
