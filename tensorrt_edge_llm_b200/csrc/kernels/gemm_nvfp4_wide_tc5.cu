@@ -383,9 +383,12 @@ static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
                        const GemmParams& p, cudaStream_t stream) {
     using Cfg = WideCfg;
     auto kern = gemm_nvfp4_wide_kernel;
-    static const int max_pairs = resident_pairs(kern, kGemmThreads, Cfg::kSmem);
+    static const int max_pairs = [&] {
+        const int n = resident_pairs(kern, kGemmThreads, Cfg::kSmem);
+        if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", n, sm_count());
+        return n;
+    }();
     if (max_pairs <= 0) return fail("gemm_nvfp4_wide: configuration");
-    if (getenv("TELB_DEBUG_CLUSTERS")) fprintf(stderr, "[telb] gemm_nvfp4_wide: %d CTA pairs can be resident (of %d SMs)\n", max_pairs, sm_count());
     const int total = p.tiles_a * p.tiles_b;
     const cudaError_t e = launch_pairs(kern, total < max_pairs ? total : max_pairs, kGemmThreads, Cfg::kSmem, stream, ta, tb, tsfa, tsfb, k64, k64, p);
     if (e != cudaSuccess) return fail("cudaLaunchKernelEx(gemm_nvfp4_wide)", e);
