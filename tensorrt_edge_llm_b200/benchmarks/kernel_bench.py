@@ -116,6 +116,7 @@ def bench_attention(args):
         else:
             cu._check(cu.lib().telb_set_decode_variant(args.variant), "set_decode_variant", 0)
     flip = [0]
+    one_tile = "tile" if args.variant >= 0 and q > 4 else None       # the variants are forms of the one-tile kernel
 
     fp8 = getattr(args, "kv_dtype", "model") == "fp8"
     if fp8:                 # E4M3 pages read in place by the decode kernel (decode-shaped steps only)
@@ -128,7 +129,7 @@ def bench_attention(args):
         if fp8:
             return cu.paged_attention_decode_fp8(q8, kv if flip[0] else kv_alt, meta, d ** -0.5, None, kv_scales, torch.bfloat16,
                                                  splits=args.splits or None)
-        return cu.paged_attention(qt, kv if flip[0] else kv_alt, meta, d ** -0.5, splits=args.splits or None)
+        return cu.paged_attention(qt, kv if flip[0] else kv_alt, meta, d ** -0.5, splits=args.splits or None, kernel=one_tile)
 
     out = fn()
     if args.check:      # numerics against the fp32 statement of the op
@@ -300,7 +301,7 @@ def main():
     a.add_argument("--q", type=int, default=1)
     a.add_argument("--hq", type=int, default=32)
     a.add_argument("--hkv", type=int, default=8)
-    a.add_argument("--variant", type=int, default=-1, help="decode kernel ring / residency variant (see telb_set_decode_variant)")
+    a.add_argument("--variant", type=int, default=-1, help="ring / residency variant of the decode kernel (up to 4 rows) or of the one-tile kernel, which then takes the step (telb_set_decode_variant, telb_set_attn_variant)")
     a.add_argument("--splits", type=int, default=0, help="KV splits (0 = heuristic)")
     a.add_argument("--check", action="store_true", help="compare with the fp32 reference first")
     a.add_argument("--kv-dtype", default="model", choices=["model", "fp8"], help="fp8: E4M3 cache pages read in place (decode shapes)")
