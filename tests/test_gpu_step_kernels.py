@@ -76,6 +76,59 @@ def test_gemm_nvfp4_tile_swiglu_equals_the_128_wide_kernel(cu, m, inter, k, dtyp
     assert torch.equal(rows[0], rows[1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,world", [(130, 256, 64, 2), (300, 544, 288, 2), (1000, 1056, 512, 4), (385, 288, 1056, 3)])
+def test_gemm_nvfp4_tile_scatters_rows_to_their_ranks(cu, m, n, k, world, dtype):
+    """The reduce-scatter form: every row leaves for its owner's buffer with the bits of the plain product, and nothing else is written.  The
+    ranks' buffers all lie on this GPU, and nothing waits."""
+    xq, xsf, wq, w_sf, alpha, extra = _nvfp4_operands(cu, m, n, k, dtype)
+    rpr, rank = -(-m // world), world - 1
+    parts = [torch.full((world * rpr, n), float("nan"), device="cuda", dtype=dtype) for _ in range(world)]
+    f = cu.GemmFusion()
+    for d in range(world):
+        f.rs_out[d] = parts[d].data_ptr()
+    f.rs_world, f.rs_rank, f.rs_rows_per_rank = world, rank, rpr
+    cu.gemm_fused(cu.QuantActs(xq, xsf, (m, k), dtype), wq, f, w_sf=w_sf, alpha=alpha, bias=extra["bias"])
+    want = cu.gemm_nvfp4(xq, xsf, wq, w_sf, alpha, dtype, bias=extra["bias"], mode=1)
+    _check_status(cu)
+    for d in range(world):
+        rows = want[d * rpr:(d + 1) * rpr]
+        assert torch.equal(parts[d][rank * rpr:rank * rpr + rows.shape[0]], rows)
+        parts[d][rank * rpr:rank * rpr + rows.shape[0]] = float("nan")
+        assert parts[d].isnan().all()
+
+
+@pytest.mark.parametrize("tokens,inter", [(600, 256), (1500, 192), (9, 256)])
+def test_grouped_swiglu_tiles_equal_the_separate_pass(cu, tokens, inter, monkeypatch):
+    """SwiGLU and quantisation in the epilogue of the 128 x 256 expert tiles, half a tile of columns at an expert's end, against the product
+    and its pass, and against the 128-wide kernel."""
+    from tensorrt_edge_llm_b200.config import QuantConfig, qwen3_30b_a3b_config
+    from tensorrt_edge_llm_b200.models.qwen3_moe import MoEBlock
+    cfg = qwen3_30b_a3b_config(num_hidden_layers=1, hidden_size=512, moe_intermediate_size=inter, num_experts=72, num_experts_per_tok=4)
+    cfg.quant = QuantConfig(quant_type="nvfp4")
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, 512, device="cuda", generator=g).bfloat16()
+    L, outs = cu.lib(), []
+    old = L.telb_set_nvfp4_wide_mode(0)
+    try:
+        for fused in ("1", "0"):
+            monkeypatch.setenv("TELB_MOE_SWIGLU_FUSION", fused)
+            blk = MoEBlock(cfg, "model.layers.0.mlp").cuda()
+            blk.random_init(torch.Generator().manual_seed(3), std=0.05)
+            blk.finalize()
+            assert blk._w13_interleaved == (fused == "1")
+            blk.input_scale.fill_(float(x.abs().max()) / (6.0 * 448.0))
+            blk.down_input_scale.fill_(0.5 / (6.0 * 448.0))
+            blk._refresh_alpha()
+            for mode in (0, 1):
+                L.telb_set_nvfp4_wide_mode(mode)
+                outs.append(blk(x))
+    finally:
+        L.telb_set_nvfp4_wide_mode(old)
+    _check_status(cu)
+    assert outs[0].abs().max() > 0 and all(torch.equal(outs[0], o) for o in outs[1:])
+
+
 def _step_meta(q_lens, pasts):
     from tensorrt_edge_llm_b200.ops import build_step_meta
     return build_step_meta(q_lens, pasts, torch.zeros(len(q_lens), 1, dtype=torch.int32), 64, slot_ids=list(range(len(q_lens)))[::-1]).to("cuda")
@@ -243,6 +296,26 @@ def test_prompt_attention_on_both_sides_of_the_route(cu, q_lens, past_lens, hq, 
     got, tile = cu.paged_attention(q, kv, meta, 128 ** -0.5), cu.paged_attention(q, kv, meta, 128 ** -0.5, kernel="tile")
     assert (got.float() - want.float()).norm() < 8e-3 * want.float().norm()
     assert torch.equal(got, tile) == one_tile
+    _check_status(cu)
+
+
+@pytest.mark.parametrize("q_lens,past_lens,hq,hkv", [([300, 90], [1000, 290], 32, 8), ([200], [333], 16, 16), ([40, 130], [120, 7], 8, 1)])
+def test_two_tile_attention_of_infinite_and_missing_scores(cu, q_lens, past_lens, hq, hkv):
+    """Scores of minus infinity weigh nothing, NaN and plus infinity spread to the rows that see them and to no other; under a window of 40
+    keys most rows find their block's first key tile masked, and most of 7 splits hold no key of theirs or none at all."""
+    q, kv, meta = _paged_step(q_lens, past_lens, hq, hkv, 64, torch.bfloat16)
+    q[:, :, 0] = q[:, :, 0].abs() + 1.0
+    for s, (ql, past) in enumerate(zip(q_lens, past_lens)):
+        for at, value in ((past // 2, -3e38), (past + ql // 3, float("nan")), (past + 2 * ql // 3, 3e38)):
+            kv[int(meta.page_table[s, at // 64]), 0, :, at % 64, 0] = value
+    q[:, :, 0] *= 4.0
+    for kw in (dict(), dict(sliding_window=40)):
+        want = ref.paged_attention(q, kv, meta, 128 ** -0.5, **kw)
+        for splits in (1, 3, 7):
+            got = cu.paged_attention(q, kv, meta, 128 ** -0.5, splits=splits, **kw)
+            assert torch.equal(got.isnan(), want.isnan()), (kw, splits)
+            ok = ~want.isnan()
+            assert ok.any() and (got[ok].float() - want[ok].float()).norm() < 8e-3 * want[ok].float().norm(), (kw, splits)
     _check_status(cu)
 
 
