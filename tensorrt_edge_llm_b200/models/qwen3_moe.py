@@ -173,11 +173,11 @@ class MoEBlock(nn.Module):
             cu = ops.cuda_ops()
             if (not self._w13_interleaved and self.inter % 64 == 0
                     and os.environ.get("TELB_MOE_SWIGLU_FUSION", "0") == "1"):
-                # Opt-in: the expert gate/up GEMM applies SwiGLU + quantisation in its epilogue (a 128-wide output tile then
-                # holds 64 gate features and the matching 64 up features).  Off by default because it measured slower on a
-                # B200: expert GEMMs have short K loops (hidden 2048 = 8 K steps), so the epilogue sits on the critical path
-                # and one row per lane leaves most lanes idle on the sparsely filled tiles of a decode step (FC1 58.6 -> 89.1 us
-                # at 32 tokens, 311 -> 398 us at 8192 tokens, Qwen3-30B-A3B shape); the separate element-wise kernel wins.
+                # Opt-in: the expert gate/up GEMM applies SwiGLU + quantisation in its epilogue (a 128-wide half of an output tile then
+                # holds 64 gate features and the matching 64 up features).  It was slower than the separate pass on 128 x 128 tiles, whose
+                # epilogue sat on the critical path of short K loops.  On the 128 x 256 tiles it is faster: Qwen3-30B-A3B shape, the block
+                # at 32 tokens 85.6 -> 83.9 us, 300: 113 -> 109, 1024: 138 -> 128, 8000: 470 -> 412.  Not the default yet: steps below about a
+                # wave of wide tiles still take the narrow ones, and are not measured.
                 self.w13.copy_(self._interleave(self.w13))
                 self.w13_scale.view(torch.uint8).copy_(self._interleave(self.w13_scale.view(torch.uint8)))
                 self.w13_alpha.copy_(self._interleave(self.w13_alpha))
